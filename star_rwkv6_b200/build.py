@@ -1,4 +1,5 @@
-"""Build the CUDA library in-tree: star_rwkv6_b200/libwkv6_b200.so (sm_100a only).
+"""Build the CUDA library in-tree: star_rwkv6_b200/libwkv6_b200.so (sm_100a only), and the native call path of the torch
+operator: star_rwkv6_b200/_native.so (csrc/wkv6_torch.cpp, host code against the installed torch).
 
 ``python star_rwkv6_b200/build.py`` (run as a script, so that it works before the library exists) compiles every ``.cu`` under ``csrc/`` with nvcc and links
 one shared object that exports the C ABI declared in ``include/wkv6_b200.h``.  nvcc
@@ -14,6 +15,7 @@ import sys
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libwkv6_b200.so")
+NATIVE = os.path.join(PKG, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -36,10 +38,24 @@ def xla_ffi_include_dir():
     return inc if os.path.exists(os.path.join(inc, "xla", "ffi", "api", "ffi.h")) else None
 
 
+def native_command():
+    """g++ line for _native.so.  torch is located without importing it; its libraries are in the process before the
+    module is (the package imports torch first), so no run path is recorded."""
+    import importlib.util
+    import sysconfig
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"] + ["-I" + d for d in inc]
+            + [os.path.join(CSRC, "wkv6_torch.cpp"), "-o", NATIVE, "-L" + os.path.join(torch_dir, "lib")]
+            + ["-l" + n for n in ("torch_python", "torch", "torch_cpu", "torch_cuda", "c10", "c10_cuda", "dl")])
+
+
 def _stale() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(NATIVE):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(NATIVE))
     deps = glob.glob(os.path.join(CSRC, "*")) + glob.glob(os.path.join(PKG, "..", "include", "*.h"))
     return any(os.path.getmtime(f) > t for f in deps)
 
@@ -62,9 +78,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc, "-x", "cu"] + flags + ["-I", inc, "-c", src, "-o", obj]
         procs.append((cmd, subprocess.Popen(cmd)))
         objs.append(obj)
+    procs.append((native_command(), subprocess.Popen(native_command())))
     for cmd, pr in procs:
         if pr.wait() != 0:
-            raise RuntimeError("nvcc failed: " + " ".join(cmd))
+            raise RuntimeError("compilation failed: " + " ".join(cmd))
     subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB] + objs + ["-lcudart"])
     return LIB
 

@@ -1,0 +1,289 @@
+// Native call path of the torch operator: what a call of RWKVKernelOperator / wkv6() does between Python and the C ABI
+// (include/wkv6_b200.h), as one C++ function per call.
+//
+// Small calls are bound by the host, not by the GPU: one decode step is 2.5 us of kernel, the parity-size training call
+// 90 us, and the same steps in Python (argument checks, a ctypes struct, tensor allocation through the dispatcher, a
+// Python autograd node with zero-filled gradients for the checkpoint buffer) took 27 us and 300 us.  Every function
+// here returns None when the call is not the plain one it handles - other tensor types, a tracing or dispatch mode,
+// layouts or arguments that need a conversion or an error message - and the Python path then runs instead.
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/grad_mode.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/csrc/Exceptions.h>
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+
+#include "../../include/wkv6_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// The library is the one the Python side loaded (WKV6_B200_LIB may select another build of it).
+struct Api {
+    decltype(&::wkv6_forward) forward = nullptr;
+    decltype(&::wkv6_backward) backward = nullptr;
+    decltype(&::wkv6_decode) decode = nullptr;
+    decltype(&::wkv6_ckpt_bytes) ckpt_bytes = nullptr;
+    decltype(&::wkv6_backward_workspace_bytes) backward_workspace_bytes = nullptr;
+    decltype(&::wkv6_sum_rows) sum_rows = nullptr;
+    decltype(&::wkv6_resolve_variant) resolve_variant = nullptr;
+    decltype(&::wkv6_last_error) last_error = nullptr;
+    bool bound = false;
+} api;
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kBFloat16: return WKV6_BF16;
+        case at::kHalf: return WKV6_F16;
+        case at::kFloat: return WKV6_F32;
+        default: return -1;
+    }
+}
+
+// fp16 inputs give fp32 outputs and gradients, as in the reference operator
+at::ScalarType result_type(at::ScalarType x) { return x == at::kHalf ? at::kFloat : x; }
+
+bool plain_mode() {
+    return api.bound && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() &&
+           !torch::jit::tracer::isTracing();
+}
+
+// A strided CUDA tensor of the exact class Tensor (or Parameter), not wrapped by a functorch transform.
+bool plain_tensor(PyObject *o) {
+    if (!THPVariable_CheckExact(o)) return false;
+    const Tensor &t = THPVariable_Unpack(o);
+    constexpr c10::DispatchKeySet odd({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+                                       c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
+                                       c10::DispatchKey::Conjugate, c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
+    return t.defined() && t.is_cuda() && t.layout() == at::kStrided && (t.key_set() & odd).empty();
+}
+
+struct Call {
+    wkv6_problem p{};
+    at::ScalarType xt{}, yt{};
+    int64_t B = 0, T = 0, C = 0, H = 0;
+    bool dense = false;
+};
+
+// Fills the problem from the operator's five tensors; false when they are not what the native path handles.
+bool make_call(const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u, int64_t N, int64_t variant,
+               Call &c) {
+    if (r.dim() != 3 || N <= 0) return false;
+    c.B = r.size(0); c.T = r.size(1); c.C = r.size(2);
+    if (c.B == 0 || c.T == 0 || c.C == 0 || c.C % N != 0) return false;
+    c.H = c.C / N;
+    c.xt = r.scalar_type();
+    c.yt = result_type(c.xt);
+    const auto dev = r.device();
+    for (const Tensor *t : {&r, &k, &v, &w})
+        if (reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) return false;
+    for (const Tensor *t : {&k, &v, &w})
+        if (t->scalar_type() != c.xt || t->device() != dev || t->sizes() != r.sizes() || t->strides() != r.strides()) return false;
+    if (u.device() != dev || (u.scalar_type() != c.xt && u.scalar_type() != at::kFloat) || u.numel() != c.C || !u.is_contiguous())
+        return false;
+    if (dtype_code(c.xt) < 0 || r.stride(2) != 1) return false;
+    c.dense = r.is_contiguous();
+    wkv6_problem &p = c.p;
+    p.B = (int32_t)c.B; p.T = (int32_t)c.T; p.H = (int32_t)c.H; p.N = (int32_t)N;
+    p.x_dtype = dtype_code(c.xt); p.y_dtype = dtype_code(c.yt); p.u_dtype = dtype_code(u.scalar_type());
+    p.gu_dtype = WKV6_F32; p.s_dtype = WKV6_F32; p.variant = (int32_t)variant;
+    p.row_stride = c.T > 1 ? r.stride(1) : c.C;
+    p.batch_stride = c.B > 1 ? r.stride(0) : c.T * p.row_stride;
+    return api.resolve_variant(&p) >= 0;
+}
+
+Tensor like(const Tensor &r, at::ScalarType t, bool dense) {   // one stride set serves inputs and outputs
+    return dense ? at::detail::empty_cuda(r.sizes(), t, r.device(), std::nullopt)
+                 : at::detail::empty_strided_cuda(r.sizes(), r.strides(), t, r.device());
+}
+
+Tensor bytes(size_t n, const Tensor &r) { return at::detail::empty_cuda({(int64_t)n}, at::kByte, r.device(), std::nullopt); }
+
+void *stream_of(const Tensor &r) { return c10::cuda::getCurrentCUDAStream(r.device().index()).stream(); }
+
+void ok(int rc) { TORCH_CHECK(rc == 0, "wkv6_b200 error ", rc, ": ", api.last_error()); }
+
+struct WKV6Function : public torch::autograd::Function<WKV6Function> {
+    static Tensor forward(AutogradContext *ctx, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w,
+                          const Tensor &u, int64_t N, int64_t variant) {
+        Call c;
+        TORCH_CHECK(make_call(r, k, v, w, u, N, variant, c), "wkv6: unsupported call");   // checked by the caller
+        Tensor y = like(r, c.yt, c.dense);
+        const size_t nckpt = api.ckpt_bytes(&c.p);
+        Tensor ckpt = bytes(nckpt, r);
+        ok(api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), nullptr, nullptr,
+                       0, nullptr, nckpt ? ckpt.data_ptr() : nullptr, stream_of(r)));
+        ctx->save_for_backward({r, k, v, w, u, ckpt});
+        ctx->saved_data["N"] = N;
+        ctx->saved_data["variant"] = variant;
+        return y;
+    }
+
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        variable_list s = ctx->get_saved_variables();
+        const Tensor &r = s[0], &k = s[1], &v = s[2], &w = s[3], &u = s[4], &ckpt = s[5];
+        const bool twice = at::GradMode::is_enabled();
+        Tensor gr, gk, gv, gw, gu;
+        {
+            at::NoGradGuard no_grad;
+            c10::cuda::CUDAGuard guard(r.device());
+            Call c;
+            TORCH_CHECK(make_call(r, k, v, w, u, ctx->saved_data["N"].toInt(), ctx->saved_data["variant"].toInt(), c),
+                        "wkv6: unsupported call");
+            Tensor gy = grads[0];
+            if (gy.strides() != r.strides() || reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 != 0)
+                gy = like(r, c.yt, c.dense).copy_(gy);
+            gr = like(r, c.yt, c.dense); gk = like(r, c.yt, c.dense);
+            gv = like(r, c.yt, c.dense); gw = like(r, c.yt, c.dense);
+            Tensor rows = at::detail::empty_cuda({c.B, c.C}, at::kFloat, r.device(), std::nullopt);
+            const bool have = ckpt.numel() > 0;
+            const size_t nws = api.backward_workspace_bytes(&c.p, have ? 1 : 0);
+            Tensor ws;
+            if (nws) ws = bytes(nws, r);
+            void *st = stream_of(r);
+            ok(api.backward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), gy.data_ptr(), gr.data_ptr(),
+                            gk.data_ptr(), gv.data_ptr(), gw.data_ptr(), rows.data_ptr(), have ? ckpt.data_ptr() : nullptr,
+                            nws ? ws.data_ptr() : nullptr, nws, st));
+            if (c.B == 1) {
+                gu = rows;
+            } else {
+                gu = at::detail::empty_cuda({c.C}, at::kFloat, r.device(), std::nullopt);
+                ok(api.sum_rows(rows.data_ptr<float>(), c.B, c.C, gu.data_ptr<float>(), st));
+            }
+            gu = gu.view(u.sizes());
+            if (gu.scalar_type() != u.scalar_type()) gu = gu.to(u.scalar_type());
+            if (c.yt != c.xt) { gr = gr.to(c.xt); gk = gk.to(c.xt); gv = gv.to(c.xt); gw = gw.to(c.xt); }
+        }
+        variable_list out{gr, gk, gv, gw, gu};
+        if (twice) {   // a gradient of the gradient is not available: say so when it is asked for
+            auto err = std::make_shared<torch::autograd::DelayedError>("the WKV6 backward is not differentiable", 5);
+            for (auto &t : out) t = t.detach().requires_grad_(true);
+            out = (*err)(std::move(out));
+        }
+        out.resize(7);
+        return out;
+    }
+};
+
+PyObject *none() { Py_RETURN_NONE; }
+
+#define ARG(i) THPVariable_Unpack(args[i])
+
+// wkv6(r, k, v, w, u, head_size, variant) -> y or None
+PyObject *py_wkv6(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 7 || !plain_mode()) return none();
+    for (int i = 0; i < 5; ++i)
+        if (!plain_tensor(args[i])) return none();
+    const int64_t N = PyLong_AsLongLong(args[5]), variant = PyLong_AsLongLong(args[6]);
+    if (PyErr_Occurred()) return nullptr;
+    const Tensor &r = ARG(0), &k = ARG(1), &v = ARG(2), &w = ARG(3), &u = ARG(4);
+    Call c;
+    if (!make_call(r, k, v, w, u, N, variant, c)) return none();
+    const bool grad = at::GradMode::is_enabled() && (r.requires_grad() || k.requires_grad() || v.requires_grad() ||
+                                                     w.requires_grad() || u.requires_grad());
+    Tensor y;
+    {
+        pybind11::gil_scoped_release no_gil;
+        c10::cuda::CUDAGuard guard(r.device());
+        if (grad) {
+            y = WKV6Function::apply(r, k, v, w, u, N, variant);
+        } else {
+            y = like(r, c.yt, c.dense);
+            if (api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), nullptr,
+                            nullptr, 0, nullptr, nullptr, stream_of(r)) != 0)
+                y.reset();
+        }
+    }
+    if (!y.defined()) return none();   // the Python path raises the library's error
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+// with_state(r, k, v, w, u, init_state or None, head_size, variant) -> (y, state) or None
+PyObject *py_with_state(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 8 || !plain_mode()) return none();
+    for (int i = 0; i < 5; ++i)
+        if (!plain_tensor(args[i])) return none();
+    const int64_t N = PyLong_AsLongLong(args[6]), variant = PyLong_AsLongLong(args[7]);
+    if (PyErr_Occurred()) return nullptr;
+    const Tensor &r = ARG(0), &k = ARG(1), &v = ARG(2), &w = ARG(3), &u = ARG(4);
+    Call c;
+    if (!make_call(r, k, v, w, u, N, variant, c)) return none();
+    const void *s_in = nullptr;
+    int32_t kinds = 0;
+    at::ScalarType st = at::kFloat;
+    if (args[5] != Py_None) {
+        if (!plain_tensor(args[5])) return none();
+        const Tensor &s = ARG(5);
+        const int64_t d = s.dim();
+        if ((d != 3 && d != 4) || !s.is_contiguous() || s.device() != r.device()) return none();
+        if (s.size(d - 3) != c.H || s.size(d - 2) != N || s.size(d - 1) != N) return none();
+        kinds = d == 4 ? (int32_t)s.size(0) : 1;
+        if (kinds != 1 && kinds != c.B) return none();
+        st = s.scalar_type();
+        if (st != at::kFloat && st != at::kBFloat16) return none();
+        s_in = s.data_ptr();
+        c.p.s_dtype = dtype_code(st);
+    }
+    Tensor y, out;
+    int rc;
+    {
+        pybind11::gil_scoped_release no_gil;
+        c10::cuda::CUDAGuard guard(r.device());
+        y = like(r, c.yt, c.dense);
+        out = at::detail::empty_cuda({c.B, c.H, N, N}, st, r.device(), std::nullopt);
+        if (c.T == 1 && N == 64 && c.dense && st == at::kFloat)   // a decode step: the state-streaming kernel
+            rc = api.decode(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(),
+                            static_cast<const float *>(s_in), nullptr, kinds, out.data_ptr<float>(), stream_of(r));
+        else
+            rc = api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), s_in, nullptr,
+                             kinds, out.data_ptr(), nullptr, stream_of(r));
+    }
+    if (rc != 0) return none();        // the Python path raises the library's error
+    PyObject *t = PyTuple_New(2);
+    if (t == nullptr) return nullptr;
+    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(y)));
+    PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(out)));
+    return t;
+    END_HANDLE_TH_ERRORS
+}
+
+// bind(path): the library's entry points, from the object the Python side has loaded
+PyObject *py_bind(PyObject *, PyObject *arg) {
+    const char *path = PyUnicode_AsUTF8(arg);
+    if (path == nullptr) return nullptr;
+    void *h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+    if (h == nullptr) return PyErr_Format(PyExc_ImportError, "%s", dlerror());
+#define SYM(name)                                                                                                   \
+    if ((api.name = reinterpret_cast<decltype(api.name)>(dlsym(h, "wkv6_" #name))) == nullptr)                      \
+        return PyErr_Format(PyExc_ImportError, "%s lacks wkv6_" #name, path);
+    SYM(forward) SYM(backward) SYM(decode) SYM(ckpt_bytes) SYM(backward_workspace_bytes) SYM(sum_rows)
+    SYM(resolve_variant) SYM(last_error)
+#undef SYM
+    api.bound = true;
+    Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"bind", py_bind, METH_O, nullptr},
+    {"wkv6", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_wkv6)), METH_FASTCALL, nullptr},
+    {"with_state", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_with_state)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }

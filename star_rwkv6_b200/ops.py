@@ -19,6 +19,13 @@ import torch
 from . import _lib
 from ._lib import BF16, F16, F32, Problem, check, lib
 
+try:
+    from . import _native  # csrc/wkv6_torch.cpp: the same calls without Python between the caller and the C ABI
+except ImportError as e:
+    raise ImportError("star_rwkv6_b200/_native.so is missing or was built against another torch: build it with "
+                      "`python star_rwkv6_b200/build.py`") from e
+_native.bind(_lib.LIB_PATH)
+
 _DT = {torch.bfloat16: BF16, torch.float16: F16, torch.float32: F32}
 
 
@@ -226,6 +233,10 @@ _forward_op.register_autograd(_autograd_backward, setup_context=_setup_context)
 
 def wkv6(r, k, v, w, u, head_size: int, variant: int = _lib.VARIANT_AUTO) -> torch.Tensor:
     """Differentiable WKV6 with a zero initial state: y[B,T,C] from r,k,v,w [B,T,C] and u [H,N]."""
+    if not torch.compiler.is_compiling():
+        y = _native.wkv6(r, k, v, w, u, head_size, variant)
+        if y is not None:
+            return y
     need_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (r, k, v, w, u))
     y, _ = torch.ops.wkv6_b200.forward(r, k, v, w, u, head_size, need_grad, variant)
     return y
@@ -235,6 +246,10 @@ def wkv6_with_state(r, k, v, w, u, head_size: int, init_state=None, state_map=No
                     variant: int = _lib.VARIANT_AUTO):
     """Forward only, with an optional initial state and the final state returned (no autograd), as the
     reference's with-state kernel (rwkv_kernel/jax_kernel/rwkv_kernels.cu:165-190)."""
+    if state_map is None and not torch.compiler.is_compiling():
+        out = _native.with_state(r, k, v, w, u, init_state, head_size, variant)
+        if out is not None:
+            return out
     with torch.no_grad():
         y, s_out, _ = forward_raw(r, k, v, w, u, head_size, s_in=init_state, s_map=state_map, want_state=True,
                                   variant=variant)

@@ -29,6 +29,16 @@ class RWKVKernelOperator:
         self.segments = segments
 
     def __call__(self, r, k, v, w, u, return_state=False, init_state=None, state_map=None):
+        if state_map is None and not torch.compiler.is_compiling():
+            # the plain calls without Python in between; None: not one of them, or arguments that need the checks below
+            if return_state:
+                out = ops._native.with_state(r, k, v, w, u, init_state, self.head_size, self.variant)
+                if out is not None:
+                    return out
+            elif init_state is None and self.segments == 1:
+                y = ops._native.wkv6(r, k, v, w, u, self.head_size, self.variant)
+                if y is not None:
+                    return y, None
         B, T, C = r.shape
         assert C % self.head_size == 0
         H = C // self.head_size
