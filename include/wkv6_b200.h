@@ -125,6 +125,27 @@ WKV6_API int wkv6_backward(const wkv6_problem *p, const void *r, const void *k, 
 WKV6_API size_t wkv6_backward_workspace_bytes(const wkv6_problem *p, int have_ckpt);
 
 /*
+ * The same forward and backward with every sequence cut into G segments that run side by side (summaries of the
+ * segments as affine maps of the state, a scan over them, then the main sweeps from the entering states): for problems
+ * with too few (batch, head) pairs to fill the GPU.  wkv6_split_segments says how many segments this problem gets on the
+ * current device (1: not split, use the calls above); results agree with the unsplit calls to rounding.
+ *   states    : wkv6_split_state_bytes(p) bytes, the segments' entering states: written by the forward, read by the backward
+ *   workspace : wkv6_split_workspace_bytes(p, 0 forward / 1 backward) bytes of device scratch
+ *   gu_rows   : fp32 [B*G, H, N]; gu is their sum over the first axis (wkv6_sum_rows)
+ * The backward of fp16 inputs is not split (WKV6_ERR_UNSUPPORTED): use wkv6_backward for it.
+ * No counterpart in the reference (its kernels walk each sequence with one block).
+ */
+WKV6_API int32_t wkv6_split_segments(const wkv6_problem *p);
+WKV6_API size_t wkv6_split_state_bytes(const wkv6_problem *p);
+WKV6_API size_t wkv6_split_workspace_bytes(const wkv6_problem *p, int backward);
+WKV6_API int wkv6_forward_split(const wkv6_problem *p, const void *r, const void *k, const void *v, const void *w,
+                                const void *u, void *y, const void *s_in, const int64_t *s_map, int32_t s_kinds,
+                                void *s_out, float *states, void *workspace, size_t workspace_bytes, void *stream);
+WKV6_API int wkv6_backward_split(const wkv6_problem *p, const void *r, const void *k, const void *v, const void *w,
+                                 const void *u, const void *gy, void *gr, void *gk, void *gv, void *gw, float *gu_rows,
+                                 const float *states, void *workspace, size_t workspace_bytes, void *stream);
+
+/*
  * Backward without any caller-provided scratch.  It has no counterpart in the reference.
  *
  * Some hosts of this library may not allocate device memory around a call and have no buffer to lend it: a

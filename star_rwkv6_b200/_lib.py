@@ -22,6 +22,7 @@ SYMBOLS = (
     "wkv6_backward", "wkv6_backward_workspace_bytes", "wkv6_backward_static_scratch", "wkv6_static_scratch_bytes",
     "wkv6_decode", "wkv6_decode_gated", "wkv6_decode_ln_shift_mix", "wkv6_decode_lora_mix", "wkv6_decode_relu_sq",
     "wkv6_decode_sigmoid_mul_add", "wkv6_softmax_xent_bf16", "wkv6_segment_summary", "wkv6_segment_summary_for_scan", "wkv6_state_scan", "wkv6_backward_seeded", "wkv6_sum_rows",
+    "wkv6_split_segments", "wkv6_split_state_bytes", "wkv6_split_workspace_bytes", "wkv6_forward_split", "wkv6_backward_split",
     "wkv6_groupnorm_gate_forward", "wkv6_groupnorm_gate_backward", "wkv6_groupnorm_gate_workspace_bytes",
     "wkv6_groupnorm_silu_gate_forward", "wkv6_groupnorm_silu_gate_backward",
     "wkv6_shift_mix_forward", "wkv6_shift_mix_backward", "wkv6_shift_mix_workspace_bytes", "wkv6_copy_2d_async",
@@ -101,6 +102,16 @@ def _load():
     lib.wkv6_backward_seeded.restype = ctypes.c_int
     lib.wkv6_backward_seeded.argtypes = [pp] + [vp] * 11 + [vp, vp, vp, sz, vp]
     i64 = ctypes.c_int64
+    lib.wkv6_split_segments.restype = i32
+    lib.wkv6_split_segments.argtypes = [pp]
+    lib.wkv6_split_state_bytes.restype = sz
+    lib.wkv6_split_state_bytes.argtypes = [pp]
+    lib.wkv6_split_workspace_bytes.restype = sz
+    lib.wkv6_split_workspace_bytes.argtypes = [pp, ctypes.c_int]
+    lib.wkv6_forward_split.restype = ctypes.c_int
+    lib.wkv6_forward_split.argtypes = [pp] + [vp] * 7 + [i64p, i32, vp, vp, vp, sz, vp]
+    lib.wkv6_backward_split.restype = ctypes.c_int
+    lib.wkv6_backward_split.argtypes = [pp] + [vp] * 13 + [sz, vp]
     lib.wkv6_groupnorm_gate_forward.restype = ctypes.c_int
     lib.wkv6_groupnorm_gate_forward.argtypes = [i64, i32, i32, i32, ctypes.c_float, vp, vp, vp, vp, vp, vp]
     lib.wkv6_groupnorm_gate_backward.restype = ctypes.c_int

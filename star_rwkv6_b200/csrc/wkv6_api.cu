@@ -169,6 +169,67 @@ int wkv6_backward(const wkv6_problem *p, const void *r, const void *k, const voi
     return seq_backward(p, d, r, k, v, w, u, gy, gr, gk, gv, gw, gu, workspace, workspace_bytes, st);
 }
 
+int32_t wkv6_split_segments(const wkv6_problem *p) {
+    Dims d;
+    int rc = validate(p, &d);
+    if (rc) return rc;
+    rc = resolve_variant(p);
+    if (rc < 0) return fail(rc, "the chunked variant does not cover this problem");
+    return rc == WKV6_VARIANT_SEQ ? seq_split_segments(p) : 1;
+}
+
+size_t wkv6_split_state_bytes(const wkv6_problem *p) {
+    const int G = wkv6_split_segments(p);
+    return G > 1 ? seq_split_state_bytes(p, G) : 0;
+}
+
+size_t wkv6_split_workspace_bytes(const wkv6_problem *p, int backward) {
+    Dims d;
+    const int G = wkv6_split_segments(p);
+    return G > 1 && validate(p, &d) == 0 ? seq_split_workspace(p, d, G, backward != 0) : 0;
+}
+
+static int check_split(const wkv6_problem *p, Dims *d, int *G, const float *states, const void *ws, size_t ws_bytes, int backward) {
+    *G = wkv6_split_segments(p);
+    if (*G < 0) return *G;
+    if (*G == 1) return fail(WKV6_ERR_INVALID, "the problem is not split (wkv6_split_segments is 1)");
+    if (int rc = validate(p, d)) return rc;
+    if (int rc = check_ptr(states, "states")) return rc;
+    if (int rc = check_ptr(ws, "workspace")) return rc;
+    const size_t need = wkv6_split_workspace_bytes(p, backward);
+    return ws_bytes >= need ? WKV6_OK : fail(WKV6_ERR_WORKSPACE, "split workspace: need %zu bytes, got %zu", need, ws_bytes);
+}
+
+int wkv6_forward_split(const wkv6_problem *p, const void *r, const void *k, const void *v, const void *w, const void *u, void *y,
+                       const void *s_in, const int64_t *s_map, int32_t s_kinds, void *s_out, float *states, void *workspace,
+                       size_t workspace_bytes, void *stream) {
+    Dims d;
+    int G;
+    if (int rc = check_split(p, &d, &G, states, workspace, workspace_bytes, 0)) return rc;
+    WKV6_CHECK_PTR(r); WKV6_CHECK_PTR(k); WKV6_CHECK_PTR(v); WKV6_CHECK_PTR(w); WKV6_CHECK_PTR(y);
+    if (u == nullptr) return fail(WKV6_ERR_INVALID, "u is NULL");
+    if (s_in == nullptr && s_map != nullptr) return fail(WKV6_ERR_INVALID, "s_map given without s_in");
+    if (s_in != nullptr && (s_kinds < 1 || s_kinds > p->B || (s_map == nullptr && s_kinds != 1 && s_kinds != p->B)))
+        return fail(WKV6_ERR_INVALID, "s_kinds=%d does not fit B=%d", s_kinds, p->B);
+    return seq_forward_split(p, d, G, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, states, static_cast<float *>(workspace),
+                             static_cast<cudaStream_t>(stream));
+}
+
+int wkv6_backward_split(const wkv6_problem *p, const void *r, const void *k, const void *v, const void *w, const void *u,
+                        const void *gy, void *gr, void *gk, void *gv, void *gw, float *gu_rows, const float *states,
+                        void *workspace, size_t workspace_bytes, void *stream) {
+    Dims d;
+    int G;
+    if (int rc = check_split(p, &d, &G, states, workspace, workspace_bytes, 1)) return rc;
+    WKV6_CHECK_PTR(r); WKV6_CHECK_PTR(k); WKV6_CHECK_PTR(v); WKV6_CHECK_PTR(w); WKV6_CHECK_PTR(gy);
+    WKV6_CHECK_PTR(gr); WKV6_CHECK_PTR(gk); WKV6_CHECK_PTR(gv); WKV6_CHECK_PTR(gw);
+    if (u == nullptr || gu_rows == nullptr) return fail(WKV6_ERR_INVALID, "u or gu_rows is NULL");
+    wkv6_problem q = *p;
+    q.gu_dtype = WKV6_F32;
+    return seq_backward_split(&q, d, G, r, k, v, w, u, gy, gr, gk, gv, gw, gu_rows, states, static_cast<float *>(workspace),
+                              static_cast<cudaStream_t>(stream));
+}
+
 int wkv6_segment_summary(const wkv6_problem *p, const void *x1, const void *x2, const void *w, int reverse,
                          float *state_out, float *dec_log2_out, void *stream) {
     Dims d;
@@ -198,7 +259,8 @@ int wkv6_state_scan(int32_t B, int32_t H, int32_t N, int32_t G, const float *dec
     if (N != 64) return fail(WKV6_ERR_UNSUPPORTED, "state scan is built for N == 64");
     if (B < 0 || H < 0 || G < 1) return fail(WKV6_ERR_INVALID, "bad B/H/G (%d,%d,%d)", B, H, G);
     if (dec_log2 == nullptr || state_sum == nullptr || state_in_out == nullptr) return fail(WKV6_ERR_INVALID, "NULL argument");
-    return chunk_state_scan(B, H, G, dec_log2, state_sum, s0, state_in_out, last_out, reverse != 0, static_cast<cudaStream_t>(stream));
+    return state_scan(B, H, G, dec_log2, state_sum, s0, nullptr, B, WKV6_F32, state_in_out, last_out, WKV6_F32, reverse != 0,
+                      static_cast<cudaStream_t>(stream));
 }
 
 int wkv6_sum_rows(const float *in, int64_t rows, int64_t n, float *out, void *stream) {

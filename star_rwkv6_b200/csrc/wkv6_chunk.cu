@@ -13,7 +13,7 @@
 namespace wkv6 {
 
 // SMs of the current device (looked up once per device).
-static int sm_count() {
+int sm_count() {
     static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
@@ -241,25 +241,35 @@ int chunk_segment_summary(const wkv6_problem *p, const Dims &d, const void *x1, 
 //   forward : S_in[g] = state entering segment g      = 2^{dec[g-1]} S_in[g-1] + b[g-1],  S_in[0] = s0 (or 0)
 //   reverse : A_in[g] = reverse state entering at the end of segment g = 2^{dec[g+1]} A_in[g+1] + b[g+1],  A_in[G-1] = 0
 // Segment g of sequence (b, h) sits at batch index b*G + g of the [B*G, H, ...] summary arrays.
-__global__ void state_scan_kernel(int B, int H, int G, const float *__restrict__ dec, const float *__restrict__ bsum,
-                                  const float *__restrict__ s0, float *__restrict__ out, float *__restrict__ last,
-                                  bool reverse) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over B*H*64*64
-    if (idx >= (size_t)B * H * 4096) return;
-    const int ij = (int)(idx & 4095), i = ij >> 6;
-    const int h = (int)((idx >> 12) % H), b = (int)(idx / ((size_t)H * 4096));
-    float s = (!reverse && s0 != nullptr) ? s0[idx] : 0.f;
+// A thread carries four neighbouring elements of one state row.
+__global__ void __launch_bounds__(128) state_scan_kernel(int B, int H, int G, const float *__restrict__ dec,
+                                                         const float *__restrict__ bsum, const void *__restrict__ s0,
+                                                         const int64_t *__restrict__ s_map, int s_kinds, int s_dtype,
+                                                         float *__restrict__ out, void *__restrict__ last, int last_dtype,
+                                                         bool reverse) {
+    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over B*H*64*16
+    if (idx >= (size_t)B * H * 1024) return;
+    const int ij = (int)(idx & 1023) * 4, i = ij >> 6;
+    const int h = (int)((idx >> 10) % H), b = (int)(idx / ((size_t)H * 1024));
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    if (!reverse && s0 != nullptr) {
+        int64_t kind = s_map ? s_map[b] : (s_kinds == 1 ? 0 : b);
+        kind = kind < 0 ? 0 : (kind >= s_kinds ? s_kinds - 1 : kind);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[e] = load_any(s0, s_dtype, ((size_t)kind * H + h) * 4096 + ij + e);
+    }
     // eight segments at a time: their loads do not depend on the running state, so they are all requested before the
     // first of them is folded in (one memory round trip per eight segments instead of one per segment)
     for (int g0 = 0; g0 < G; g0 += 8) {
-        float d8[8], b8[8];
+        float d8[8];
+        float4 b8[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const int gg = g0 + e;
             if (gg < G) {
                 const size_t seq = ((size_t)(b * G + (reverse ? G - 1 - gg : gg)) * H + h);
                 d8[e] = dec[seq * 64 + i];
-                b8[e] = bsum[seq * 4096 + ij];
+                b8[e] = *reinterpret_cast<const float4 *>(bsum + seq * 4096 + ij);
             }
         }
 #pragma unroll
@@ -267,19 +277,25 @@ __global__ void state_scan_kernel(int B, int H, int G, const float *__restrict__
             const int gg = g0 + e;
             if (gg < G) {
                 const size_t seq = ((size_t)(b * G + (reverse ? G - 1 - gg : gg)) * H + h);
-                out[seq * 4096 + ij] = s;
-                s = fmaf(exp2f(d8[e]), s, b8[e]);
+                *reinterpret_cast<float4 *>(out + seq * 4096 + ij) = make_float4(s[0], s[1], s[2], s[3]);
+                const float d = exp2f(d8[e]);
+                s[0] = fmaf(d, s[0], b8[e].x); s[1] = fmaf(d, s[1], b8[e].y);
+                s[2] = fmaf(d, s[2], b8[e].z); s[3] = fmaf(d, s[3], b8[e].w);
             }
         }
     }
-    if (last != nullptr) last[idx] = s;
+    if (last != nullptr) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) store_any(last, last_dtype, ((size_t)b * H + h) * 4096 + ij + e, s[e]);
+    }
 }
 
-int chunk_state_scan(int B, int H, int G, const float *dec, const float *bsum, const float *s0, float *out, float *last,
-                     bool reverse, cudaStream_t st) {
-    const size_t n = (size_t)B * H * 4096;
+int state_scan(int B, int H, int G, const float *dec, const float *bsum, const void *s0, const int64_t *s_map, int s_kinds,
+               int s_dtype, float *out, void *last, int last_dtype, bool reverse, cudaStream_t st) {
+    const size_t n = (size_t)B * H * 1024;
     if (n == 0 || G <= 0) return WKV6_OK;
-    state_scan_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(B, H, G, dec, bsum, s0, out, last, reverse);
+    state_scan_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(B, H, G, dec, bsum, s0, s_map, s_kinds, s_dtype, out, last,
+                                                                   last_dtype, reverse);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "state_scan_kernel launch");
 }

@@ -36,6 +36,11 @@ struct Api {
     decltype(&::wkv6_ckpt_bytes) ckpt_bytes = nullptr;
     decltype(&::wkv6_backward_workspace_bytes) backward_workspace_bytes = nullptr;
     decltype(&::wkv6_sum_rows) sum_rows = nullptr;
+    decltype(&::wkv6_split_segments) split_segments = nullptr;
+    decltype(&::wkv6_split_state_bytes) split_state_bytes = nullptr;
+    decltype(&::wkv6_split_workspace_bytes) split_workspace_bytes = nullptr;
+    decltype(&::wkv6_forward_split) forward_split = nullptr;
+    decltype(&::wkv6_backward_split) backward_split = nullptr;
     decltype(&::wkv6_resolve_variant) resolve_variant = nullptr;
     decltype(&::wkv6_last_error) last_error = nullptr;
     bool bound = false;
@@ -73,6 +78,8 @@ struct Call {
     at::ScalarType xt{}, yt{};
     int64_t B = 0, T = 0, C = 0, H = 0;
     bool dense = false;
+    int G = 1;               // segments the library cuts the sequences into
+    int backward_G() const { return xt == at::kHalf ? 1 : G; }   // the backward of fp16 inputs is not split
 };
 
 // Fills the problem from the operator's five tensors; false when they are not what the native path handles.
@@ -99,7 +106,9 @@ bool make_call(const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &
     p.gu_dtype = WKV6_F32; p.s_dtype = WKV6_F32; p.variant = (int32_t)variant;
     p.row_stride = c.T > 1 ? r.stride(1) : c.C;
     p.batch_stride = c.B > 1 ? r.stride(0) : c.T * p.row_stride;
-    return api.resolve_variant(&p) >= 0;
+    if (api.resolve_variant(&p) < 0) return false;
+    c.G = api.split_segments(&p);
+    return true;
 }
 
 Tensor like(const Tensor &r, at::ScalarType t, bool dense) {   // one stride set serves inputs and outputs
@@ -111,6 +120,20 @@ Tensor bytes(size_t n, const Tensor &r) { return at::detail::empty_cuda({(int64_
 
 void *stream_of(const Tensor &r) { return c10::cuda::getCurrentCUDAStream(r.device().index()).stream(); }
 
+// The forward without a checkpoint, split where the library says so; `states` receives the segments' entering states.
+int run_forward(const Call &c, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u, Tensor &y,
+                const void *s_in, int32_t kinds, void *s_out, Tensor *states) {
+    if (c.G == 1)
+        return api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), s_in, nullptr,
+                           kinds, s_out, nullptr, stream_of(r));
+    Tensor st = bytes(api.split_state_bytes(&c.p), r);
+    const size_t nws = api.split_workspace_bytes(&c.p, 0);
+    Tensor ws = bytes(nws, r);
+    if (states) *states = st;
+    return api.forward_split(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), s_in, nullptr,
+                             kinds, s_out, static_cast<float *>(st.data_ptr()), ws.data_ptr(), nws, stream_of(r));
+}
+
 void ok(int rc) { TORCH_CHECK(rc == 0, "wkv6_b200 error ", rc, ": ", api.last_error()); }
 
 struct WKV6Function : public torch::autograd::Function<WKV6Function> {
@@ -119,11 +142,18 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
         Call c;
         TORCH_CHECK(make_call(r, k, v, w, u, N, variant, c), "wkv6: unsupported call");   // checked by the caller
         Tensor y = like(r, c.yt, c.dense);
-        const size_t nckpt = api.ckpt_bytes(&c.p);
-        Tensor ckpt = bytes(nckpt, r);
-        ok(api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), nullptr, nullptr,
-                       0, nullptr, nckpt ? ckpt.data_ptr() : nullptr, stream_of(r)));
-        ctx->save_for_backward({r, k, v, w, u, ckpt});
+        // what the backward needs beside the inputs: the chunk checkpoints, or the segments' entering states
+        Tensor kept;
+        if (c.G > 1) {
+            ok(run_forward(c, r, k, v, w, u, y, nullptr, 0, nullptr, &kept));
+            if (c.backward_G() == 1) kept = bytes(0, r);
+        } else {
+            const size_t nckpt = api.ckpt_bytes(&c.p);
+            kept = bytes(nckpt, r);
+            ok(api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), nullptr, nullptr,
+                           0, nullptr, nckpt ? kept.data_ptr() : nullptr, stream_of(r)));
+        }
+        ctx->save_for_backward({r, k, v, w, u, kept});
         ctx->saved_data["N"] = N;
         ctx->saved_data["variant"] = variant;
         return y;
@@ -131,7 +161,7 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
 
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         variable_list s = ctx->get_saved_variables();
-        const Tensor &r = s[0], &k = s[1], &v = s[2], &w = s[3], &u = s[4], &ckpt = s[5];
+        const Tensor &r = s[0], &k = s[1], &v = s[2], &w = s[3], &u = s[4], &kept = s[5];
         const bool twice = at::GradMode::is_enabled();
         Tensor gr, gk, gv, gw, gu;
         {
@@ -145,20 +175,27 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
                 gy = like(r, c.yt, c.dense).copy_(gy);
             gr = like(r, c.yt, c.dense); gk = like(r, c.yt, c.dense);
             gv = like(r, c.yt, c.dense); gw = like(r, c.yt, c.dense);
-            Tensor rows = at::detail::empty_cuda({c.B, c.C}, at::kFloat, r.device(), std::nullopt);
-            const bool have = ckpt.numel() > 0;
-            const size_t nws = api.backward_workspace_bytes(&c.p, have ? 1 : 0);
+            const int G = c.backward_G();
+            const int64_t nrows = c.B * G;
+            Tensor rows = at::detail::empty_cuda({nrows, c.C}, at::kFloat, r.device(), std::nullopt);
+            const bool have = kept.numel() > 0;
+            const size_t nws = G > 1 ? api.split_workspace_bytes(&c.p, 1) : api.backward_workspace_bytes(&c.p, have ? 1 : 0);
             Tensor ws;
             if (nws) ws = bytes(nws, r);
-            void *st = stream_of(r);
-            ok(api.backward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), gy.data_ptr(), gr.data_ptr(),
-                            gk.data_ptr(), gv.data_ptr(), gw.data_ptr(), rows.data_ptr(), have ? ckpt.data_ptr() : nullptr,
-                            nws ? ws.data_ptr() : nullptr, nws, st));
-            if (c.B == 1) {
+            void *pws = nws ? ws.data_ptr() : nullptr, *st = stream_of(r);
+            if (G > 1)
+                ok(api.backward_split(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), gy.data_ptr(),
+                                      gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gw.data_ptr(), rows.data_ptr<float>(),
+                                      static_cast<const float *>(kept.data_ptr()), pws, nws, st));
+            else
+                ok(api.backward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), gy.data_ptr(), gr.data_ptr(),
+                                gk.data_ptr(), gv.data_ptr(), gw.data_ptr(), rows.data_ptr(), have ? kept.data_ptr() : nullptr, pws,
+                                nws, st));
+            if (nrows == 1) {
                 gu = rows;
             } else {
                 gu = at::detail::empty_cuda({c.C}, at::kFloat, r.device(), std::nullopt);
-                ok(api.sum_rows(rows.data_ptr<float>(), c.B, c.C, gu.data_ptr<float>(), st));
+                ok(api.sum_rows(rows.data_ptr<float>(), nrows, c.C, gu.data_ptr<float>(), st));
             }
             gu = gu.view(u.sizes());
             if (gu.scalar_type() != u.scalar_type()) gu = gu.to(u.scalar_type());
@@ -200,8 +237,7 @@ PyObject *py_wkv6(PyObject *, PyObject *const *args, Py_ssize_t n) {
             y = WKV6Function::apply(r, k, v, w, u, N, variant);
         } else {
             y = like(r, c.yt, c.dense);
-            if (api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), nullptr,
-                            nullptr, 0, nullptr, nullptr, stream_of(r)) != 0)
+            if (run_forward(c, r, k, v, w, u, y, nullptr, 0, nullptr, nullptr) != 0)
                 y.reset();
         }
     }
@@ -248,8 +284,7 @@ PyObject *py_with_state(PyObject *, PyObject *const *args, Py_ssize_t n) {
             rc = api.decode(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(),
                             static_cast<const float *>(s_in), nullptr, kinds, out.data_ptr<float>(), stream_of(r));
         else
-            rc = api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), s_in, nullptr,
-                             kinds, out.data_ptr(), nullptr, stream_of(r));
+            rc = run_forward(c, r, k, v, w, u, y, s_in, kinds, out.data_ptr(), nullptr);
     }
     if (rc != 0) return none();        // the Python path raises the library's error
     PyObject *t = PyTuple_New(2);
@@ -270,6 +305,7 @@ PyObject *py_bind(PyObject *, PyObject *arg) {
     if ((api.name = reinterpret_cast<decltype(api.name)>(dlsym(h, "wkv6_" #name))) == nullptr)                      \
         return PyErr_Format(PyExc_ImportError, "%s lacks wkv6_" #name, path);
     SYM(forward) SYM(backward) SYM(decode) SYM(ckpt_bytes) SYM(backward_workspace_bytes) SYM(sum_rows)
+    SYM(split_segments) SYM(split_state_bytes) SYM(split_workspace_bytes) SYM(forward_split) SYM(backward_split)
     SYM(resolve_variant) SYM(last_error)
 #undef SYM
     api.bound = true;
