@@ -226,6 +226,10 @@ WKV6_API int wkv6_decode_sigmoid_mul_add(int64_t n, int32_t dtype, const void *x
 WKV6_API int wkv6_softmax_xent_bf16(int64_t rows, int32_t V, void *logits_inout, const int64_t *targets, float scale,
                                     float *loss, void *stream);
 
+/* g <- g * (*scale) in place over n bf16 values (n a multiple of 8), scale one fp32 value on the device (rounded to bf16
+ * first): the chain rule behind the loss above.  Touches nothing when the factor is 1. */
+WKV6_API int wkv6_scale_bf16(int64_t n, void *g, const float *scale, void *stream);
+
 /*
  * Sequence splitting along T (no counterpart in the reference, whose kernels cap T at a compile-time constant and
  * never split a sequence; sequences of 131072 tokens need it).  A sequence cut into G segments is

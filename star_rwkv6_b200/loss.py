@@ -33,7 +33,10 @@ class _LMLoss(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         (g,) = ctx.saved_tensors
-        return g.mul_(grad_out.to(g.dtype)).view(ctx.shape), None   # in place: the buffer is this function's own
+        scale = grad_out.to(torch.float32)
+        with torch.cuda.device(g.device):      # in place: the buffer is this function's own; nothing moves for a factor of 1
+            check(lib.wkv6_scale_bf16(g.numel(), _ptr(g), _ptr(scale), _stream(g.device)))
+        return g.view(ctx.shape), None
 
 
 def lm_loss(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
