@@ -129,7 +129,9 @@ WKV6_API size_t wkv6_backward_workspace_bytes(const wkv6_problem *p, int have_ck
  * segments as affine maps of the state, a scan over them, then the main sweeps from the entering states): for problems
  * with too few (batch, head) pairs to fill the GPU.  wkv6_split_segments says how many segments this problem gets on the
  * current device (1: not split, use the calls above); results agree with the unsplit calls to rounding.
- *   states    : wkv6_split_state_bytes(p) bytes, the segments' entering states: written by the forward, read by the backward
+ *   states    : wkv6_split_state_bytes(p) bytes: written by the forward, read by the backward.  Sequential variant: the
+ *               segments' entering states.  Chunked variant: the checkpoints of wkv6_forward (same size and contents), which
+ *               the forward leaves out when `states` is NULL.
  *   workspace : wkv6_split_workspace_bytes(p, 0 forward / 1 backward) bytes of device scratch
  *   gu_rows   : fp32 [B*G, H, N]; gu is their sum over the first axis (wkv6_sum_rows)
  * The backward of fp16 inputs is not split (WKV6_ERR_UNSUPPORTED): use wkv6_backward for it.

@@ -175,18 +175,20 @@ int32_t wkv6_split_segments(const wkv6_problem *p) {
     if (rc) return rc;
     rc = resolve_variant(p);
     if (rc < 0) return fail(rc, "the chunked variant does not cover this problem");
-    return rc == WKV6_VARIANT_SEQ ? seq_split_segments(p) : 1;
+    return rc == WKV6_VARIANT_SEQ ? seq_split_segments(p) : chunk_split_segments(p);
 }
 
 size_t wkv6_split_state_bytes(const wkv6_problem *p) {
     const int G = wkv6_split_segments(p);
-    return G > 1 ? seq_split_state_bytes(p, G) : 0;
+    if (G <= 1) return 0;
+    return resolve_variant(p) == WKV6_VARIANT_CHUNK ? chunk_ckpt_bytes(p) : seq_split_state_bytes(p, G);
 }
 
 size_t wkv6_split_workspace_bytes(const wkv6_problem *p, int backward) {
     Dims d;
     const int G = wkv6_split_segments(p);
-    return G > 1 && validate(p, &d) == 0 ? seq_split_workspace(p, d, G, backward != 0) : 0;
+    if (G <= 1 || validate(p, &d) != 0) return 0;
+    return resolve_variant(p) == WKV6_VARIANT_CHUNK ? chunk_split_workspace(p, backward != 0) : seq_split_workspace(p, d, G, backward != 0);
 }
 
 static int check_split(const wkv6_problem *p, Dims *d, int *G, const float *states, const void *ws, size_t ws_bytes, int backward) {
@@ -194,7 +196,9 @@ static int check_split(const wkv6_problem *p, Dims *d, int *G, const float *stat
     if (*G < 0) return *G;
     if (*G == 1) return fail(WKV6_ERR_INVALID, "the problem is not split (wkv6_split_segments is 1)");
     if (int rc = validate(p, d)) return rc;
-    if (int rc = check_ptr(states, "states")) return rc;
+    // the forward of the chunked variant leaves its checkpoints out when there is nowhere to put them
+    if (states != nullptr || backward || resolve_variant(p) != WKV6_VARIANT_CHUNK)
+        if (int rc = check_ptr(states, "states")) return rc;
     if (int rc = check_ptr(ws, "workspace")) return rc;
     const size_t need = wkv6_split_workspace_bytes(p, backward);
     return ws_bytes >= need ? WKV6_OK : fail(WKV6_ERR_WORKSPACE, "split workspace: need %zu bytes, got %zu", need, ws_bytes);
@@ -211,6 +215,9 @@ int wkv6_forward_split(const wkv6_problem *p, const void *r, const void *k, cons
     if (s_in == nullptr && s_map != nullptr) return fail(WKV6_ERR_INVALID, "s_map given without s_in");
     if (s_in != nullptr && (s_kinds < 1 || s_kinds > p->B || (s_map == nullptr && s_kinds != 1 && s_kinds != p->B)))
         return fail(WKV6_ERR_INVALID, "s_kinds=%d does not fit B=%d", s_kinds, p->B);
+    if (resolve_variant(p) == WKV6_VARIANT_CHUNK)
+        return chunk_forward_split(p, d, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, states, static_cast<float *>(workspace),
+                                   static_cast<cudaStream_t>(stream));
     return seq_forward_split(p, d, G, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, states, static_cast<float *>(workspace),
                              static_cast<cudaStream_t>(stream));
 }
@@ -224,6 +231,9 @@ int wkv6_backward_split(const wkv6_problem *p, const void *r, const void *k, con
     WKV6_CHECK_PTR(r); WKV6_CHECK_PTR(k); WKV6_CHECK_PTR(v); WKV6_CHECK_PTR(w); WKV6_CHECK_PTR(gy);
     WKV6_CHECK_PTR(gr); WKV6_CHECK_PTR(gk); WKV6_CHECK_PTR(gv); WKV6_CHECK_PTR(gw);
     if (u == nullptr || gu_rows == nullptr) return fail(WKV6_ERR_INVALID, "u or gu_rows is NULL");
+    if (resolve_variant(p) == WKV6_VARIANT_CHUNK)
+        return chunk_backward_split(p, d, r, k, v, w, u, gy, gr, gk, gv, gw, gu_rows, states, static_cast<float *>(workspace),
+                                    static_cast<cudaStream_t>(stream));
     wkv6_problem q = *p;
     q.gu_dtype = WKV6_F32;
     return seq_backward_split(&q, d, G, r, k, v, w, u, gy, gr, gk, gv, gw, gu_rows, states, static_cast<float *>(workspace),

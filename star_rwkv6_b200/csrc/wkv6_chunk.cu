@@ -118,9 +118,75 @@ size_t chunk_ckpt_bytes(const wkv6_problem *p) {
     return (size_t)p->B * p->H * nchunks * 4096 * sizeof(__nv_bfloat16);
 }
 
-int chunk_forward(const wkv6_problem *p, const Dims &d, const void *r, const void *k, const void *v, const void *w,
-                  const void *u, void *y, const void *s_in, const int64_t *s_map, int s_kinds, void *s_out,
-                  void *ckpt, cudaStream_t st) {
+static int chunks_of(const wkv6_problem *p) { return (p->T + kChunk - 1) / kChunk; }
+
+// What the main kernels fold into the states their segments enter with (b == NULL: nothing).
+struct Fold { const float *b = nullptr, *dec = nullptr; int sub = 0, lo = 0, pieces = 0; };
+
+// One segment: the whole sequence.
+static SegGeom whole(const wkv6_problem *p) { return SegGeom{1, chunks_of(p), chunks_of(p), 0, false}; }
+
+// How a sequence is cut along T so that two CTAs run on every SM (they share it best: a chunk of the forward takes 2.6 us on
+// an SM of its own and 3.05 us beside another CTA, one of the backward 5.2 and 7.6 us).  A segment that does not start at the end
+// its state comes from needs the summaries of the segments before it, 40 % (forward) or 20 % (backward) of a main chunk's time each.
+//   up to one sequence per SM : equal segments, as many as fill the slots, but no more than the time to read the summaries
+//                               (0.5 us each) is worth: G^2 <= 8 chunks (4 sequences of 256 chunks: 145 us with 32
+//                               segments, 155 with 64, 173 with 16)
+//   up to two per SM          : two segments.  The long one of every sequence starts with the launch; the short ones, for which the
+//                               state is known without a summary, run in the slots left free, `waves` after one another.
+// Short sequences stay whole: the summary launch costs about 4 us.
+// The summary kernel has four slots per SM: a segment is summarised in `sub` pieces of four chunks or more where that fills them.
+struct Split {
+    SegGeom seg, pieces;      // of the main kernel; of the summaries (pieces.g0: the first one needed)
+    int sub, lo;              // pieces per segment; backward: the segment g needs the pieces lo + g sub and later
+    int summaries;            // pieces that are needed
+};
+
+static Split split_geom(const wkv6_problem *p, bool backward) {
+    const int64_t seqs = (int64_t)p->B * p->H, sms = sm_count(), slots = 2 * sms;
+    const int n = chunks_of(p);
+    Split s{whole(p), whole(p), 1, 1, 0};
+    if (seqs == 0 || seqs >= slots || n < 4) return s;
+    if (seqs <= sms) {
+        int64_t G = slots / seqs;
+        while (G > 1 && G * G > 8 * (int64_t)n) --G;
+        if (G > n) G = n;
+        if (G < 2) return s;
+        int64_t sub = 4 * sms / ((G - 1) * seqs);
+        const int len = (int)((n + G - 1) / G);
+        while (sub > 1 && (4 * sub > len || G * sub * G * sub > 8 * (int64_t)n)) --sub;
+        if (sub < 1) sub = 1;
+        s.sub = s.lo = (int)sub;
+        s.pieces.first = s.pieces.rest = (int)((len + sub - 1) / sub);
+        s.pieces.G = (n + s.pieces.rest - 1) / s.pieces.rest;
+        s.seg.first = s.seg.rest = s.sub * s.pieces.rest;
+        s.seg.G = (n + s.seg.rest - 1) / s.seg.rest;
+        s.summaries = backward ? s.pieces.G - s.sub : (s.seg.G - 1) * s.sub;
+        s.pieces.g0 = backward ? s.sub : 0;
+    } else {
+        const int64_t waves = (seqs + slots - seqs - 1) / (slots - seqs);
+        int e = (int)(n / (waves + 1));
+        if (e < 4) return s;
+        s.sub = (int)(4 * sms / seqs);       // 2 or 3
+        s.pieces.rest = e / s.sub;
+        e = s.sub * s.pieces.rest;
+        s.seg.G = 2;
+        s.seg.first = backward ? n - e : e;
+        s.seg.rest = backward ? e : n - e;
+        s.seg.last_first = !backward;
+        s.pieces.first = backward ? n - e : s.pieces.rest;
+        s.pieces.G = backward ? 1 + s.sub : s.sub;
+        s.pieces.g0 = backward ? 1 : 0;
+        s.summaries = s.sub;
+    }
+    return s;
+}
+
+int chunk_split_segments(const wkv6_problem *p) { return split_geom(p, false).seg.G; }
+
+static int launch_forward(const wkv6_problem *p, const Dims &d, const SegGeom &seg, const Fold &fold,
+                          const void *r, const void *k, const void *v, const void *w, const void *u, void *y, const void *s_in,
+                          const int64_t *s_map, int s_kinds, void *s_out, void *ckpt, cudaStream_t st) {
     CUtensorMap mr, mk, mv, mw, my;
     int rc;
     if ((rc = make_map(&mr, r, p, d, "r"))) return rc;
@@ -132,19 +198,37 @@ int chunk_forward(const wkv6_problem *p, const Dims &d, const void *r, const voi
     a.u = u; a.u_dtype = p->u_dtype; a.s_in = s_in; a.s_map = s_map; a.s_kinds = s_kinds; a.s_dtype = p->s_dtype;
     a.s_out = s_out; a.write_y = (y != nullptr); a.ckpt = static_cast<__nv_bfloat16 *>(ckpt);
     a.reverse_state = false; a.dec_out = nullptr; a.B = p->B; a.T = p->T; a.H = p->H;
+    a.seg = seg; a.fold_b = fold.b; a.fold_dec = fold.dec; a.fold_sub = fold.sub;
     a.skip_load_chunk = g_skip_load_chunk.load() + 1;
     cudaError_t e = cudaFuncSetAttribute(chunk_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          ChunkFwdSmem::kAlloc);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chunk_fwd_kernel)");
-    chunk_fwd_kernel<<<p->B * p->H, 256, ChunkFwdSmem::kAlloc, st>>>(mr, mk, mv, mw, my, a);
-    e = cudaGetLastError();
+    const unsigned grid = (unsigned)(seg.G * p->B * p->H);
+    if (fold.b != nullptr) {
+        e = launch_behind(chunk_fwd_kernel, grid, 256, ChunkFwdSmem::kAlloc, st, mr, mk, mv, mw, my, a);
+    } else {
+        chunk_fwd_kernel<<<grid, 256, ChunkFwdSmem::kAlloc, st>>>(mr, mk, mv, mw, my, a);
+        e = cudaGetLastError();
+    }
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "chunk_fwd_kernel launch");
+}
+
+int chunk_forward(const wkv6_problem *p, const Dims &d, const void *r, const void *k, const void *v, const void *w,
+                  const void *u, void *y, const void *s_in, const int64_t *s_map, int s_kinds, void *s_out,
+                  void *ckpt, cudaStream_t st) {
+    return launch_forward(p, d, whole(p), Fold{}, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, ckpt, st);
 }
 
 // Workspace of the backward: one word per sequence for the hand-over between the fast and the general kernel, then,
 // without a checkpoint buffer from the forward, room for the chunk-start states, which the backward first rebuilds
 // with the forward kernel (its y output suppressed).
-static size_t flag_bytes(const wkv6_problem *p) { return (((size_t)p->B * p->H * sizeof(int)) + 255) & ~(size_t)255; }
+static size_t flag_bytes(const wkv6_problem *p, int G = 1) {
+    return (((size_t)G * p->B * p->H * sizeof(int)) + 255) & ~(size_t)255;
+}
+static int launch_backward(const wkv6_problem *p, const Dims &d, const SegGeom &seg, const Fold &fold,
+                           const void *r, const void *k, const void *v, const void *w, const void *u, const void *gy, void *gr,
+                           void *gk, void *gv, void *gw, void *gu, int gu_dtype, const void *ckpt, const float *ab_in, int *flags,
+                           cudaStream_t st);
 size_t chunk_backward_workspace(const wkv6_problem *p, const Dims &, int have_ckpt) {
     return flag_bytes(p) + (have_ckpt ? 0 : chunk_ckpt_bytes(p));
 }
@@ -169,6 +253,14 @@ int chunk_backward_seeded(const wkv6_problem *p, const Dims &d, const void *r, c
         if ((rc = chunk_forward(p, d, r, k, v, w, u, nullptr, nullptr, nullptr, 0, nullptr, area, st))) return rc;
         ckpt = area;
     }
+    return launch_backward(p, d, whole(p), Fold{}, r, k, v, w, u, gy, gr, gk, gv, gw, gu, p->gu_dtype, ckpt, ab_in, flags, st);
+}
+
+static int launch_backward(const wkv6_problem *p, const Dims &d, const SegGeom &seg, const Fold &fold,
+                           const void *r, const void *k, const void *v, const void *w, const void *u, const void *gy, void *gr,
+                           void *gk, void *gv, void *gw, void *gu, int gu_dtype, const void *ckpt, const float *ab_in, int *flags,
+                           cudaStream_t st) {
+    int rc;
     CUtensorMap mr, mk, mv, mw, mgy, mgr, mgk, mgv, mgw;
     if ((rc = make_map(&mr, r, p, d, "r"))) return rc;
     if ((rc = make_map(&mk, k, p, d, "k"))) return rc;
@@ -180,10 +272,13 @@ int chunk_backward_seeded(const wkv6_problem *p, const Dims &d, const void *r, c
     if ((rc = make_map(&mgv, gv, p, d, "gv"))) return rc;
     if ((rc = make_map(&mgw, gw, p, d, "gw"))) return rc;
     ChunkBwdArgs a{};
-    a.u = u; a.u_dtype = p->u_dtype; a.gu = gu; a.gu_dtype = p->gu_dtype;
+    a.u = u; a.u_dtype = p->u_dtype; a.gu = gu; a.gu_dtype = gu_dtype;
     a.ckpt = static_cast<const __nv_bfloat16 *>(ckpt); a.B = p->B; a.T = p->T; a.H = p->H;
     a.ab_in = ab_in; a.zero_init = (ab_in == nullptr);  // a seeded call is one segment of a longer sequence
     a.flags = flags;
+    a.seg = seg; a.fold_b = fold.b; a.fold_dec = fold.dec; a.fold_sub = fold.sub; a.fold_lo = fold.lo; a.fold_pieces = fold.pieces;
+    const int64_t blocks = (int64_t)seg.G * p->B * p->H;
+    const unsigned grid = (unsigned)blocks;
     cudaError_t e;
     if (flags != nullptr) {  // the fast kernel first; it marks the sequences it has to leave to the general one
         if (p->T % 16 == 0) {  // adjacent tokens per thread (see the kernel)
@@ -199,27 +294,33 @@ int chunk_backward_seeded(const wkv6_problem *p, const Dims &d, const void *r, c
             if ((rc = make_map_paired(&pgw, gw, p, d, "gw"))) return rc;
             e = cudaFuncSetAttribute(chunk_bwd_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideBwdSmem::kAlloc);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chunk_bwd_wide_kernel)");
-            chunk_bwd_wide_kernel<true><<<p->B * p->H, 256, WideBwdSmem::kAlloc, st>>>(pr, pk, pv, pw, pgy, pgr, pgk, pgv, pgw, a);
+            if (fold.b != nullptr)
+                e = launch_behind(chunk_bwd_wide_kernel<true>, grid, 256, WideBwdSmem::kAlloc, st, pr, pk, pv, pw, pgy, pgr, pgk, pgv, pgw, a);
+            else
+                chunk_bwd_wide_kernel<true><<<grid, 256, WideBwdSmem::kAlloc, st>>>(pr, pk, pv, pw, pgy, pgr, pgk, pgv, pgw, a);
         } else {
             e = cudaFuncSetAttribute(chunk_bwd_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideBwdSmem::kAlloc);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chunk_bwd_wide_kernel)");
-            chunk_bwd_wide_kernel<false><<<p->B * p->H, 256, WideBwdSmem::kAlloc, st>>>(mr, mk, mv, mw, mgy, mgr, mgk, mgv, mgw, a);
+            if (fold.b != nullptr)
+                e = launch_behind(chunk_bwd_wide_kernel<false>, grid, 256, WideBwdSmem::kAlloc, st, mr, mk, mv, mw, mgy, mgr, mgk, mgv, mgw, a);
+            else
+                chunk_bwd_wide_kernel<false><<<grid, 256, WideBwdSmem::kAlloc, st>>>(mr, mk, mv, mw, mgy, mgr, mgk, mgv, mgw, a);
         }
-        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "chunk_bwd_wide_kernel launch");
     }
-    auto general = (int64_t)p->B * p->H <= sm_count() ? chunk_bwd_kernel<1> : chunk_bwd_kernel<2>;
+    auto general = blocks <= sm_count() ? chunk_bwd_kernel<1> : chunk_bwd_kernel<2>;
     e = cudaFuncSetAttribute(general, cudaFuncAttributeMaxDynamicSharedMemorySize, ChunkBwdSmem::kAlloc);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chunk_bwd_kernel)");
-    e = launch_behind(general, (unsigned)(p->B * p->H), 256, ChunkBwdSmem::kAlloc, st, mr, mk, mv, mw, mgy, mgr, mgk, mgv, mgw, a);
+    e = launch_behind(general, grid, 256, ChunkBwdSmem::kAlloc, st, mr, mk, mv, mw, mgy, mgr, mgk, mgv, mgw, a);
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "chunk_bwd_kernel launch");
 }
 
 // Summary of every sequence as an affine map of the state: log2 of the total decay per key channel and the state
 // the sequence builds from zero.  Forward direction: x1 = k, x2 = v.  Reverse direction (the backward's state):
 // x1 = r, x2 = gy.  A kernel of its own (wkv6_chunk_summary.cuh): one scaled operand and one product per chunk.
-int chunk_segment_summary(const wkv6_problem *p, const Dims &d, const void *x1, const void *x2, const void *w,
-                          bool reverse, float *b_out, float *dec_log2_out, int skip_mod, int skip_rem, cudaStream_t st) {
+static int launch_summary(const wkv6_problem *p, const Dims &d, const SegGeom &seg, unsigned grid, const void *x1, const void *x2,
+                          const void *w, bool reverse, float *b_out, float *dec_log2_out, int skip_mod, int skip_rem, cudaStream_t st) {
     CUtensorMap m1, m2, mw;
     int rc;
     if ((rc = make_map(&m1, x1, p, d, "x1"))) return rc;
@@ -228,13 +329,51 @@ int chunk_segment_summary(const wkv6_problem *p, const Dims &d, const void *x1, 
     ChunkFwdArgs a{};
     a.u = nullptr; a.u_dtype = WKV6_F32; a.s_dtype = WKV6_F32; a.s_out = b_out; a.B = p->B; a.T = p->T; a.H = p->H;
     a.write_y = false; a.reverse_state = reverse; a.dec_out = dec_log2_out;
-    a.skip_mod = skip_mod; a.skip_rem = skip_rem;
+    a.skip_mod = skip_mod; a.skip_rem = skip_rem; a.seg = seg;
     cudaError_t e = cudaFuncSetAttribute(chunk_summary_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          ChunkSumSmem::kAlloc);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chunk_summary_kernel)");
-    chunk_summary_kernel<<<p->B * p->H, 256, ChunkSumSmem::kAlloc, st>>>(m1, m2, mw, a);
+    chunk_summary_kernel<<<grid, 256, ChunkSumSmem::kAlloc, st>>>(m1, m2, mw, a);
     e = cudaGetLastError();
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "chunk_summary_kernel launch");
+}
+
+int chunk_segment_summary(const wkv6_problem *p, const Dims &d, const void *x1, const void *x2, const void *w,
+                          bool reverse, float *b_out, float *dec_log2_out, int skip_mod, int skip_rem, cudaStream_t st) {
+    return launch_summary(p, d, whole(p), (unsigned)(p->B * p->H), x1, x2, w, reverse, b_out, dec_log2_out, skip_mod, skip_rem, st);
+}
+
+// Forward and backward of a problem that split_geom cuts: the summaries of the segments whose state others enter with, then
+// the main kernel, whose CTAs fold the summaries they need themselves (a scan kernel between the two cost one more launch).  The
+// checkpoints are those of the uncut forward.  Workspace: the summaries ([G][B*H] states and decays), backward: the flags behind.
+static size_t summary_floats(const wkv6_problem *p, const Split &s) { return (size_t)s.pieces.G * p->B * p->H * (4096 + 64); }
+
+size_t chunk_split_workspace(const wkv6_problem *p, bool backward) {
+    const Split s = split_geom(p, backward);
+    return summary_floats(p, s) * sizeof(float) + (backward ? flag_bytes(p, s.seg.G) : 0);
+}
+
+int chunk_forward_split(const wkv6_problem *p, const Dims &d, const void *r, const void *k, const void *v, const void *w,
+                        const void *u, void *y, const void *s_in, const int64_t *s_map, int s_kinds, void *s_out, void *ckpt,
+                        float *ws, cudaStream_t st) {
+    const Split s = split_geom(p, false);
+    const size_t seqs = (size_t)p->B * p->H;
+    const Fold f{ws, ws + s.pieces.G * seqs * 4096, s.sub, s.lo, s.pieces.G};
+    if (int rc = launch_summary(p, d, s.pieces, (unsigned)(s.summaries * seqs), k, v, w, false, ws, ws + s.pieces.G * seqs * 4096, 0, 0, st))
+        return rc;
+    return launch_forward(p, d, s.seg, f, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, ckpt, st);
+}
+
+int chunk_backward_split(const wkv6_problem *p, const Dims &d, const void *r, const void *k, const void *v, const void *w,
+                         const void *u, const void *gy, void *gr, void *gk, void *gv, void *gw, float *gu_rows, const void *ckpt,
+                         float *ws, cudaStream_t st) {
+    const Split s = split_geom(p, true);
+    const size_t seqs = (size_t)p->B * p->H;
+    const Fold f{ws, ws + s.pieces.G * seqs * 4096, s.sub, s.lo, s.pieces.G};
+    int *flags = reinterpret_cast<int *>(ws + summary_floats(p, s));
+    if (int rc = launch_summary(p, d, s.pieces, (unsigned)(s.summaries * seqs), r, gy, w, true, ws, ws + s.pieces.G * seqs * 4096, 0, 0, st))
+        return rc;
+    return launch_backward(p, d, s.seg, f, r, k, v, w, u, gy, gr, gk, gv, gw, gu_rows, WKV6_F32, ckpt, nullptr, flags, st);
 }
 
 // Exclusive scan of affine state maps over the G segments of each sequence:

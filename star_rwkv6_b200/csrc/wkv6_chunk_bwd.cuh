@@ -71,9 +71,12 @@ struct ChunkBwdSmem {
 
 struct ChunkBwdArgs {
     const void *u; int u_dtype;
-    void *gu; int gu_dtype;
+    void *gu; int gu_dtype;   // [G][B][H][64]
     const __nv_bfloat16 *ckpt;
     const float *ab_in;  // optional [B*H][64][64]: reverse state entering at the end of the sequence (zero if NULL)
+    SegGeom seg;
+    const float *fold_b, *fold_dec;  // reverse summaries of the pieces behind this segment ([fold_pieces][B*H]); NULL: one segment
+    int fold_sub, fold_lo, fold_pieces;  // segment g needs the pieces fold_lo + g fold_sub and later
     bool zero_init;      // the forward started from a zero state: gw at t = 0 is exactly zero
     int B, T, H;
     // Hand-over between the two backward kernels, one word per (batch, head) sequence: chunk_bwd_wide_kernel writes
@@ -215,8 +218,9 @@ __global__ void __launch_bounds__(256, MINB) chunk_bwd_kernel(const __grid_const
     const int w4 = warp & 3, half = warp >> 2, n0 = 4 * half;
     const int r0 = lane >> 2, q = lane & 3;
     const int ta = 16 * w4 + r0;  // this thread's rows: ta and ta + 8
-    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
-    const int nchunks = (a.T + kChunk - 1) / kChunk;
+    const SegPlace pl = seg_place(a.seg, a.B, a.T, a.H);
+    const int b = pl.b, h = pl.h, cend = pl.cend;
+    const int nchunks = cend - pl.c0;
 
     if (tid == 0) {
         mbar_init(bar_full, 1);
@@ -242,6 +246,13 @@ __global__ void __launch_bounds__(256, MINB) chunk_bwd_kernel(const __grid_const
             const int i = ta + (e >= 2 ? 8 : 0);
             AB[4 * nn + e] = a.ab_in ? a.ab_in[(size_t)blockIdx.x * 4096 + (size_t)i * 64 + j0 + (e & 1)] : 0.f;
         }
+    }
+    if (a.fold_b != nullptr)
+        fold_segments(AB, a.fold_b, a.fold_dec, (int64_t)(a.fold_pieces - 1) * pl.seqs + pl.seq, -pl.seqs,
+                      a.fold_pieces - a.fold_lo - pl.g * a.fold_sub, ta, 8 * n0 + 2 * q);
+#pragma unroll
+    for (int nn = 0; nn < 4; ++nn) {
+        const int j0 = 8 * (n0 + nn) + 2 * q;
         *reinterpret_cast<uint32_t *>(sAB + sw128_off(ta, j0)) = pack_bf2(AB[4 * nn], AB[4 * nn + 1]);
         *reinterpret_cast<uint32_t *>(sAB + sw128_off(ta + 8, j0)) = pack_bf2(AB[4 * nn + 2], AB[4 * nn + 3]);
     }
@@ -275,9 +286,9 @@ __global__ void __launch_bounds__(256, MINB) chunk_bwd_kernel(const __grid_const
         mbar_expect_tx(bar_late, 3 * kTile);
         tma_load_3d(sV, &tm_v, bar_late, h * 64, c * kChunk, b);
         tma_load_3d(sG, &tm_gy, bar_late, h * 64, c * kChunk, b);
-        bulk_load(sS, a.ckpt + ((size_t)blockIdx.x * nchunks + c) * 4096, kTile, bar_late);
+        bulk_load(sS, a.ckpt + ((size_t)pl.seq * pl.total + c) * 4096, kTile, bar_late);
     };
-    if (tid == 0) issue_loads(nchunks - 1);
+    if (tid == 0) issue_loads(cend - 1);
 
     constexpr uint32_t idKK = umma_idesc_bf16(64, 64, false, false);
     constexpr uint32_t idKK96 = umma_idesc_bf16(64, 96, false, false);
@@ -298,7 +309,7 @@ __global__ void __launch_bounds__(256, MINB) chunk_bwd_kernel(const __grid_const
     bool pend_full = true, pend_late = true;
     uint32_t pend_parity = 0;
     for (int it = 0; it < nchunks; ++it) {
-        const int c = nchunks - 1 - it;
+        const int c = cend - 1 - it;
         WKV6_TSTAMP(it, 0);
         if (!cta_wait(bar_full, it & 1, warp)) err = 1;
         if (tid == 0) pend_full = false;
@@ -613,7 +624,7 @@ __global__ void __launch_bounds__(256, MINB) chunk_bwd_kernel(const __grid_const
         tc_fence_after_sync();
         WKV6_TSTAMP(it, 9);
         // every input tile is dead once the second MMA group has completed: fetch the next chunk now
-        if (tid == 0 && c > 0 && err == 0) {
+        if (tid == 0 && it + 1 < nchunks && err == 0) {
             issue_loads(c - 1);
             pend_full = pend_late = true;
             pend_parity = (uint32_t)(it + 1) & 1u;

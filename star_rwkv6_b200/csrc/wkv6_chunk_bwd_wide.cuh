@@ -123,8 +123,9 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
     const int w4 = warp & 3, half = warp >> 2, n0 = 4 * half;
     const int r0 = lane >> 2, q = lane & 3;
     const int ta = 16 * w4 + r0;  // this thread's rows: ta and ta + 8
-    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
-    const int nchunks = (a.T + kChunk - 1) / kChunk;
+    const SegPlace pl = seg_place(a.seg, a.B, a.T, a.H);
+    const int b = pl.b, h = pl.h, cend = pl.cend;
+    const int nchunks = cend - pl.c0;
     WKV6_CSTAMP(0);
 
     if (tid == 0) {
@@ -175,17 +176,17 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
         else tma_store_3d(m, src, h * 64, c * kChunk, b);
     };
     auto issue_early = [&](int c) {  // tiles that are dead once the second MMA group has completed
-        par_early = (uint32_t)(nchunks - 1 - c) & 1u;
+        par_early = (uint32_t)(cend - 1 - c) & 1u;
         mbar_expect_tx(bar_w, kTile);
         ld_tile(sW, &tm_w, bar_w, c);
         mbar_expect_tx(bar_late, 3 * kTile);
         ld_tile(sV, &tm_v, bar_late, c);
         ld_tile(sG, &tm_gy, bar_late, c);
-        bulk_load(sS, a.ckpt + ((size_t)blockIdx.x * nchunks + c) * 4096, kTile, bar_late);
+        bulk_load(sS, a.ckpt + ((size_t)pl.seq * pl.total + c) * 4096, kTile, bar_late);
         pend_w = pend_late = true;
     };
     auto issue_rk = [&](int c) {  // tiles the second epilogue still reads
-        par_rk = (uint32_t)(nchunks - 1 - c) & 1u;
+        par_rk = (uint32_t)(cend - 1 - c) & 1u;
         mbar_expect_tx(bar_rk, 2 * kTile);
         ld_tile(sR, &tm_r, bar_rk, c);
         ld_tile(sK, &tm_k, bar_rk, c);
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
     // Copies are issued by one thread of warp 4, so that warps 0-3, whose first lanes issue the MMAs, never
     // queue behind them.
     const bool copy_thread = (tid == 128);
-    if (copy_thread) { issue_early(nchunks - 1); issue_rk(nchunks - 1); }
+    if (copy_thread) { issue_early(cend - 1); issue_rk(cend - 1); }
 
     // the reverse state entering at the end of the sequence: fp32 copy in tensor memory, bf16 operand copy in shared memory
     {
@@ -207,6 +208,16 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
                 const int i = ta + (e >= 2 ? 8 : 0);
                 AB[4 * nn + e] = a.ab_in ? a.ab_in[(size_t)blockIdx.x * 4096 + (size_t)i * 64 + j0 + (e & 1)] : 0.f;
             }
+        }
+        if (a.fold_b != nullptr && pl.g + 1 < a.seg.G) {
+            // launched behind the summary kernel with programmatic serialization: nothing before this point reads what that
+            // kernel writes or writes what it reads
+            grid_dependency_wait();
+            fold_segments(AB, a.fold_b, a.fold_dec, (int64_t)(a.fold_pieces - 1) * pl.seqs + pl.seq, -pl.seqs,
+                          a.fold_pieces - a.fold_lo - pl.g * a.fold_sub, ta, 8 * n0 + 2 * q);
+        }
+#pragma unroll
+        for (int nn = 0; nn < 4; ++nn) {
             *reinterpret_cast<uint32_t *>(sAB + FO(nn, 0)) = pack_bf2(AB[4 * nn], AB[4 * nn + 1]);
             *reinterpret_cast<uint32_t *>(sAB + FO(nn, 1)) = pack_bf2(AB[4 * nn + 2], AB[4 * nn + 3]);
         }
@@ -238,7 +249,7 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
     int err = 0;
     bool bail = false;  // a chunk beyond the single-reference limit: leave this sequence to the general kernel
     for (int it = 0; it < nchunks; ++it) {
-        const int c = nchunks - 1 - it;
+        const int c = cend - 1 - it;
         WKV6_TSTAMP(it, 0);
         if (!cta_wait(bar_w, it & 1, warp)) err = 1;
         if (copy_thread) pend_w = false;
@@ -531,7 +542,7 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
         tc_fence_after_sync();
         WKV6_TSTAMP(it, 9);
         // w, v, gy and the state tile are dead once the second MMA group has completed: fetch the next chunk's now
-        if (copy_thread && c > 0 && err == 0) issue_early(c - 1);
+        if (copy_thread && it + 1 < nchunks && err == 0) issue_early(c - 1);
 
         // ---- epilogue 2: gr, gk, gv, gw, one 8-column repetition at a time
         float loc[16];  // G minus its per-channel base (see below)
@@ -643,7 +654,7 @@ __global__ void __launch_bounds__(256, 2) chunk_bwd_wide_kernel(const __grid_con
         __syncthreads();
         WKV6_TSTAMP(it, 10);
         // every thread has read its raw r, k: fetch the next chunk's
-        if (copy_thread && c > 0 && err == 0) issue_rk(c - 1);
+        if (copy_thread && it + 1 < nchunks && err == 0) issue_rk(c - 1);
         // G_t = e^{c_63} <S_in, Abar> + sum_all b + sum_{later blocks} q + (suffix_incl(q) - a)_t ;  gw = -exp(w) G.
         // The part that is the same for all tokens of a block is formed once per (block, channel) by one thread.
         {

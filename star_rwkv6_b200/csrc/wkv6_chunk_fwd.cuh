@@ -88,9 +88,78 @@ struct ChunkFwdSmem {
     static constexpr int kAlloc = kBytes;
 };
 
+// How the sequences are cut along T: segment 0 has `first` chunks, the others `rest` (the last one what is left).  The grid
+// holds the segments segment-major; `last_first` starts it with the last segment (the longest one runs from the start of
+// the launch), `g0` leaves out the ones before g0.
+struct SegGeom {
+    int G, first, rest;
+    int g0;
+    bool last_first;
+};
+
+struct SegPlace {      // what one CTA works on
+    int b, h, g;
+    int c0, cend;      // its chunks
+    int total;         // chunks of the whole sequence
+    int seq, seqs;     // b * H + h of B * H
+};
+
+__device__ __forceinline__ SegPlace seg_place(const SegGeom &s, int B, int T, int H) {
+    SegPlace p;
+    p.seqs = B * H;
+    const int gi = (int)blockIdx.x / p.seqs;
+    p.seq = (int)blockIdx.x - gi * p.seqs;
+    p.b = p.seq / H;
+    p.h = p.seq - p.b * H;
+    p.g = s.last_first ? s.G - 1 - gi : s.g0 + gi;
+    p.total = (T + kChunk - 1) / kChunk;
+    p.c0 = p.g == 0 ? 0 : s.first + (p.g - 1) * s.rest;
+    p.cend = min(p.total, p.g == 0 ? s.first : p.c0 + s.rest);
+    return p;
+}
+
+// Entering state of a segment from the summaries of the n pieces between it and the end the state comes from: S <- 2^dec S + b,
+// nearest to that end first (index `at`, then `at` + step, ...).  S is this thread's accumulator fragment (rows ta, ta + 8, columns
+// col + 8 nn, + 1).  The loads do not depend on the running state: four pieces are requested at a time.
+__device__ __forceinline__ void fold_segments(float (&S)[16], const float *bsum, const float *dec, int64_t at, int64_t step, int n,
+                                              int ta, int col) {
+#pragma unroll 1
+    for (int e0 = 0; e0 < n; e0 += 4) {
+        float2 x[4][8];
+        float d[4][2];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (e0 + e < n) {
+                const float *p = bsum + (at + (e0 + e) * step) * 4096 + ta * 64 + col;
+                const float *pd = dec + (at + (e0 + e) * step) * 64 + ta;
+                d[e][0] = __ldcg(pd); d[e][1] = __ldcg(pd + 8);   // not the read-only path: written while this kernel was resident
+#pragma unroll
+                for (int nn = 0; nn < 4; ++nn) {
+                    x[e][2 * nn] = __ldcg(reinterpret_cast<const float2 *>(p + 8 * nn));
+                    x[e][2 * nn + 1] = __ldcg(reinterpret_cast<const float2 *>(p + 8 * 64 + 8 * nn));
+                }
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (e0 + e < n) {
+                const float d0 = exp2f(d[e][0]), d1 = exp2f(d[e][1]);
+#pragma unroll
+                for (int nn = 0; nn < 4; ++nn) {
+                    S[4 * nn] = fmaf(d0, S[4 * nn], x[e][2 * nn].x);
+                    S[4 * nn + 1] = fmaf(d0, S[4 * nn + 1], x[e][2 * nn].y);
+                    S[4 * nn + 2] = fmaf(d1, S[4 * nn + 2], x[e][2 * nn + 1].x);
+                    S[4 * nn + 3] = fmaf(d1, S[4 * nn + 3], x[e][2 * nn + 1].y);
+                }
+            }
+    }
+}
+
 struct ChunkFwdArgs {
     const void *u; int u_dtype;
     const void *s_in; const int64_t *s_map; int s_kinds; int s_dtype; void *s_out;
+    SegGeom seg;
+    const float *fold_b, *fold_dec;  // summaries of the pieces before this segment ([pieces][B*H]); NULL: one segment
+    int fold_sub;                    // pieces per segment
     __nv_bfloat16 *ckpt;  // optional [B*H][T/64][64*64] bf16 chunk-start states in operand (swizzled) layout
     int B, T, H;
     bool write_y;         // false: only states / checkpoints are produced
@@ -183,8 +252,9 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     const int w4 = warp & 3, half = warp >> 2, n0 = 4 * half;
     const int q = lane & 3, r0 = lane >> 2;
     const int ta = 16 * w4 + r0;
-    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
-    const int nchunks = (a.T + kChunk - 1) / kChunk;
+    const SegPlace pl = seg_place(a.seg, a.B, a.T, a.H);
+    const int b = pl.b, h = pl.h, c0 = pl.c0;
+    const int nchunks = pl.cend - c0;
     WKV6_CSTAMP(0);
 
     if (tid == 0) {
@@ -209,8 +279,8 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     const int load_slot = (lane == 0 && warp >= 2 && warp <= 5) ? warp - 2 : -1;  // 0..3 = r, k, v, w
     const int skip_chunk = a.skip_load_chunk - 1;  // test hook, -1 in normal use
     auto issue_loads = [&](int ic2) {  // every thread calls it; the four loading threads act
-        if (load_slot < 0 || ic2 == skip_chunk) return;
-        const int c = ic2;
+        const int c = c0 + ic2;
+        if (load_slot < 0 || c == skip_chunk) return;
         const int st = ic2 & 1;
         uint8_t *dst = smem + st * SM::kStage + load_slot * kTile;
         const CUtensorMap *tm = load_slot == 0 ? &tm_r : load_slot == 1 ? &tm_k : load_slot == 2 ? &tm_v : &tm_w;
@@ -258,6 +328,12 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
                 }
             }
         }
+        if (a.fold_b != nullptr && pl.g > 0) {
+            // launched behind the summary kernel with programmatic serialization: nothing before this point reads what that
+            // kernel writes or writes what it reads
+            grid_dependency_wait();
+            fold_segments(S, a.fold_b, a.fold_dec, pl.seq, pl.seqs, pl.g * a.fold_sub, ta, 8 * n0 + 2 * q);
+        }
 #pragma unroll
         for (int nn = 0; nn < 4; ++nn) {
             const int j = 8 * (n0 + nn) + 2 * q;
@@ -288,8 +364,8 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
 
     const bool copy_thread = (tid == 32);
     if (copy_thread) {
-        if (a.ckpt != nullptr) {  // state at the start of chunk 0, already in operand layout
-            bulk_store(a.ckpt + (size_t)blockIdx.x * nchunks * 4096, sSB, kTile);
+        if (a.ckpt != nullptr) {  // state at the start of the first chunk, already in operand layout
+            bulk_store(a.ckpt + ((size_t)pl.seq * pl.total + c0) * 4096, sSB, kTile);
             bulk_commit();
         }
     }
@@ -317,7 +393,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     float2 x[8];
     auto pass1 = [&](int ic1) {
         const uint8_t *wt = smem + (ic1 & 1) * SM::kStage + 3 * kTile + tofs;
-        const bool full_chunk = (ic1 + 1) * kChunk <= a.T;
+        const bool full_chunk = (c0 + ic1 + 1) * kChunk <= a.T;
         float2 cs = make_float2(0.f, 0.f);
 #pragma unroll
         for (int tt = 0; tt < 8; ++tt) {
@@ -326,7 +402,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
             float2 l2 = mul2(make_float2(ex2f(e2.x), ex2f(e2.y)), make_float2(-kLog2e, -kLog2e));
             l2.x = fmaxf(l2.x, kMinLogDecay2);
             l2.y = fmaxf(l2.y, kMinLogDecay2);
-            if (!full_chunk && ic1 * kChunk + 16 * w4 + 8 * half + tt >= a.T) l2 = make_float2(0.f, 0.f);
+            if (!full_chunk && (c0 + ic1) * kChunk + 16 * w4 + 8 * half + tt >= a.T) l2 = make_float2(0.f, 0.f);
             cs = add2(cs, l2);
             x[tt] = cs;
         }
@@ -340,7 +416,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
 
     WKV6_CSTAMP(5);
     for (int ic = 0; ic < nchunks && err == 0; ++ic) {
-        const int c = ic;  // chunk processed in this iteration
+        const int c = c0 + ic;  // chunk processed in this iteration
         const int st = ic & 1;
         uint8_t *sR = smem + st * SM::kStage;  // this stage: r, k, v, w tiles at +0, +kTile, +2 kTile, +3 kTile
         const uint64_t so = (uint64_t)(st * (SM::kStage >> 4));
@@ -598,8 +674,8 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
         } else if (copy_thread) {
             // the state entering the next chunk is complete in shared memory: checkpoint it for the backward.
             // Its read is drained (bulk_wait_read) before the next chunk's first barrier, ahead of the rewrite.
-            if (a.ckpt != nullptr && c + 1 < nchunks) {
-                bulk_store(a.ckpt + ((size_t)blockIdx.x * nchunks + c + 1) * 4096, sSB, kTile);
+            if (a.ckpt != nullptr && ic + 1 < nchunks) {
+                bulk_store(a.ckpt + ((size_t)pl.seq * pl.total + c + 1) * 4096, sSB, kTile);
                 bulk_commit();
             }
         }
@@ -642,14 +718,14 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     if (err != 0 && load_slot >= 0) {
         // loads still in flight target this CTA's shared memory: wait for them (bounded) before leaving
         for (int ic2 = loads_consumed; ic2 < loads_issued; ++ic2)
-            if (ic2 != skip_chunk) mbar_wait(&bar_full[ic2 & 1], (ic2 >> 1) & 1);
+            if (c0 + ic2 != skip_chunk) mbar_wait(&bar_full[ic2 & 1], (ic2 >> 1) & 1);
     }
     if (copy_thread) {
         if (err != 0) atomicExch(&g_chunk_status, err);
         bulk_wait<0>();
     }
-    if (err == 0 && a.s_out != nullptr) {
-        const size_t so2 = (size_t)blockIdx.x * 4096;
+    if (err == 0 && a.s_out != nullptr && pl.cend == pl.total) {
+        const size_t so2 = (size_t)pl.seq * 4096;
 #pragma unroll
         for (int nn = 0; nn < 4; ++nn)
 #pragma unroll

@@ -25,7 +25,9 @@ struct ChunkSumSmem {
     static constexpr int kAlloc = kBytes;
 };
 
-__global__ void __launch_bounds__(256, 2) chunk_summary_kernel(const __grid_constant__ CUtensorMap tm_x1,
+// Four CTAs per SM (64 registers, 51 KB each): a chunk is one chain of load, exponentials, product and fold, and with two of them
+// per SM the kernel read 4.2 TB/s.
+__global__ void __launch_bounds__(256, 4) chunk_summary_kernel(const __grid_constant__ CUtensorMap tm_x1,
                                                                const __grid_constant__ CUtensorMap tm_x2,
                                                                const __grid_constant__ CUtensorMap tm_w,
                                                                const ChunkFwdArgs a) {
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(256, 2) chunk_summary_kernel(const __grid_cons
         if (threadIdx.x == 0) atomicExch(&g_chunk_status, 50);
         return;
     }
+    launch_dependents();  // the main kernel of a split call may be scheduled from now on (it waits before it reads the summaries)
     // a segment whose summary the caller's scan never reads (the last of a sequence going forward, the first in reverse)
     if (a.skip_mod > 0 && (int)(blockIdx.x / a.H) % a.skip_mod == a.skip_rem) return;
     float *sHead = reinterpret_cast<float *>(smem + SM::oHead);
@@ -51,8 +54,10 @@ __global__ void __launch_bounds__(256, 2) chunk_summary_kernel(const __grid_cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int w4 = warp & 3, half = warp >> 2, n0 = 4 * half;
     const int ta = 16 * w4 + (lane >> 2);
-    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
-    const int nchunks = (a.T + kChunk - 1) / kChunk;
+    const SegPlace pl = seg_place(a.seg, a.B, a.T, a.H);
+    const int b = pl.b, h = pl.h;
+    const int nchunks = pl.cend - pl.c0;
+    const size_t row = (size_t)pl.g * pl.seqs + pl.seq;  // of the summary arrays
 
     if (tid == 0) {
         mbar_init(&bar_full[0], 3);  // one arrival per loading thread
@@ -77,7 +82,7 @@ __global__ void __launch_bounds__(256, 2) chunk_summary_kernel(const __grid_cons
     const int load_slot = (lane == 0 && warp >= 2 && warp <= 4) ? warp - 2 : -1;  // 0..2 = x1, x2, w
     auto issue_loads = [&](int ic2) {  // every thread calls it; the three loading threads act
         if (load_slot < 0) return;
-        const int c = a.reverse_state ? nchunks - 1 - ic2 : ic2;
+        const int c = a.reverse_state ? pl.cend - 1 - ic2 : pl.c0 + ic2;
         const int st = ic2 & 1;
         uint8_t *dst = smem + st * SM::kStage + load_slot * kTile;
         const CUtensorMap *tm = load_slot == 0 ? &tm_x1 : load_slot == 1 ? &tm_x2 : &tm_w;
@@ -94,7 +99,7 @@ __global__ void __launch_bounds__(256, 2) chunk_summary_kernel(const __grid_cons
     int loads_issued = (nchunks > 1) ? 2 : 1, loads_consumed = 0;
     float2 dsum = make_float2(0.f, 0.f);  // warp 0: log2 of the decay accumulated over all chunks, channels 2*lane, +1
     for (int ic = 0; ic < nchunks; ++ic) {
-        const int c = a.reverse_state ? nchunks - 1 - ic : ic;
+        const int c = a.reverse_state ? pl.cend - 1 - ic : pl.c0 + ic;
         const int st = ic & 1;
         uint8_t *sX = smem + st * SM::kStage;
         const uint64_t so = (uint64_t)(st * (SM::kStage >> 4));
@@ -197,9 +202,9 @@ __global__ void __launch_bounds__(256, 2) chunk_summary_kernel(const __grid_cons
     }
     if (tid == 32 && err != 0) atomicExch(&g_chunk_status, 300 + err);
     if (err == 0 && a.dec_out != nullptr && warp == 0)
-        *reinterpret_cast<float2 *>(a.dec_out + (size_t)blockIdx.x * 64 + 2 * lane) = dsum;
+        *reinterpret_cast<float2 *>(a.dec_out + row * 64 + 2 * lane) = dsum;
     if (err == 0 && a.s_out != nullptr) {
-        float *out = static_cast<float *>(a.s_out) + (size_t)blockIdx.x * 4096;
+        float *out = static_cast<float *>(a.s_out) + row * 4096;
         const int q = lane & 3;
 #pragma unroll
         for (int nn = 0; nn < 4; ++nn) {

@@ -63,6 +63,15 @@ int chunk_segment_summary(const wkv6_problem *p, const Dims &d, const void *x1, 
                           bool reverse, float *b_out, float *dec_log2_out, int skip_mod, int skip_rem, cudaStream_t st);
 int state_scan(int B, int H, int G, const float *dec, const float *bsum, const void *s0, const int64_t *s_map, int s_kinds,
                int s_dtype, float *out, void *last, int last_dtype, bool reverse, cudaStream_t st);
+// Sequences cut along T into G segments, for problems that leave SMs idle otherwise (1: not cut).
+int chunk_split_segments(const wkv6_problem *p);
+size_t chunk_split_workspace(const wkv6_problem *p, bool backward);
+int chunk_forward_split(const wkv6_problem *p, const Dims &d, const void *r, const void *k, const void *v, const void *w,
+                        const void *u, void *y, const void *s_in, const int64_t *s_map, int s_kinds, void *s_out, void *ckpt,
+                        float *ws, cudaStream_t st);
+int chunk_backward_split(const wkv6_problem *p, const Dims &d, const void *r, const void *k, const void *v, const void *w,
+                         const void *u, const void *gy, void *gr, void *gk, void *gv, void *gw, float *gu_rows, const void *ckpt,
+                         float *ws, cudaStream_t st);
 int resolve_variant(const wkv6_problem *p);
 
 }  // namespace wkv6

@@ -77,7 +77,7 @@ struct Call {
     wkv6_problem p{};
     at::ScalarType xt{}, yt{};
     int64_t B = 0, T = 0, C = 0, H = 0;
-    bool dense = false;
+    bool dense = false, chunked = false;
     int G = 1;               // segments the library cuts the sequences into
     int backward_G() const { return xt == at::kHalf ? 1 : G; }   // the backward of fp16 inputs is not split
 };
@@ -106,7 +106,9 @@ bool make_call(const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &
     p.gu_dtype = WKV6_F32; p.s_dtype = WKV6_F32; p.variant = (int32_t)variant;
     p.row_stride = c.T > 1 ? r.stride(1) : c.C;
     p.batch_stride = c.B > 1 ? r.stride(0) : c.T * p.row_stride;
-    if (api.resolve_variant(&p) < 0) return false;
+    const int variant_of = api.resolve_variant(&p);
+    if (variant_of < 0) return false;
+    c.chunked = variant_of == WKV6_VARIANT_CHUNK;
     c.G = api.split_segments(&p);
     return true;
 }
@@ -126,12 +128,13 @@ int run_forward(const Call &c, const Tensor &r, const Tensor &k, const Tensor &v
     if (c.G == 1)
         return api.forward(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), s_in, nullptr,
                            kinds, s_out, nullptr, stream_of(r));
-    Tensor st = bytes(api.split_state_bytes(&c.p), r);
+    Tensor st;   // the chunked variant needs it for a backward only
+    if (states || !c.chunked) st = bytes(api.split_state_bytes(&c.p), r);
     const size_t nws = api.split_workspace_bytes(&c.p, 0);
     Tensor ws = bytes(nws, r);
     if (states) *states = st;
     return api.forward_split(&c.p, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), s_in, nullptr,
-                             kinds, s_out, static_cast<float *>(st.data_ptr()), ws.data_ptr(), nws, stream_of(r));
+                             kinds, s_out, st.defined() ? static_cast<float *>(st.data_ptr()) : nullptr, ws.data_ptr(), nws, stream_of(r));
 }
 
 void ok(int rc) { TORCH_CHECK(rc == 0, "wkv6_b200 error ", rc, ": ", api.last_error()); }

@@ -21,8 +21,8 @@ from .. import _lib, ops
 
 class RWKVKernelOperator:
     def __init__(self, head_size, max_sequence_length=None, variant="auto", segments=1):
-        """``segments``: 1 = one kernel walks each (batch, head) sequence; an integer G > 1 or "auto" cuts every
-        sequence into G pieces along T that run concurrently (worth it when B*H is small; bf16, head size 64)."""
+        """``segments``: an integer G > 1 cuts every sequence into G pieces along T that run concurrently (bf16, head size
+        64); 1 and "auto" leave it to the library, which cuts where B*H sequences would leave SMs idle."""
         self.head_size = int(head_size)
         self.max_sequence_length = max_sequence_length
         self.variant = _lib.VARIANTS[variant] if isinstance(variant, str) else int(variant)
@@ -35,7 +35,7 @@ class RWKVKernelOperator:
                 out = ops._native.with_state(r, k, v, w, u, init_state, self.head_size, self.variant)
                 if out is not None:
                     return out
-            elif init_state is None and self.segments == 1:
+            elif init_state is None and self.segments in (1, "auto"):
                 y = ops._native.wkv6(r, k, v, w, u, self.head_size, self.variant)
                 if y is not None:
                     return y, None
