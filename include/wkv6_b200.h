@@ -133,7 +133,8 @@ WKV6_API size_t wkv6_backward_workspace_bytes(const wkv6_problem *p, int have_ck
  *               segments' entering states.  Chunked variant: the checkpoints of wkv6_forward (same size and contents), which
  *               the forward leaves out when `states` is NULL.
  *   workspace : wkv6_split_workspace_bytes(p, 0 forward / 1 backward) bytes of device scratch
- *   gu_rows   : fp32 [B*G, H, N]; gu is their sum over the first axis (wkv6_sum_rows)
+ *   gu_rows   : fp32 [B*G, H, N]; gu is their sum over the first axis (wkv6_sum_rows).  Order: [B][G] (sequential variant) or
+ *               [G][B] (chunked variant)
  * The backward of fp16 inputs is not split (WKV6_ERR_UNSUPPORTED): use wkv6_backward for it.
  * No counterpart in the reference (its kernels walk each sequence with one block).
  */
