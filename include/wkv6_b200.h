@@ -317,6 +317,27 @@ WKV6_API int wkv6_shift_mix_backward(int32_t B, int32_t T, int32_t C, int32_t dt
                                      size_t workspace_bytes, void *stream);
 WKV6_API size_t wkv6_shift_mix_workspace_bytes(int32_t B, int32_t T, int32_t C, int32_t m_is_vector);
 
+/* Two vector mixes of the same x (the channel-mix block's, rwkv6_model.py:66-71) in one pass; backward: one gx for both, and
+ * wkv6_shift_mix_workspace_bytes(B,T,C,2) bytes of scratch. */
+WKV6_API int wkv6_shift_mix_pair_forward(int32_t B, int32_t T, int32_t C, int32_t dtype, const void *x, const float *mu0,
+                                         const float *mu1, void *out0, void *out1, void *stream);
+WKV6_API int wkv6_shift_mix_pair_backward(int32_t B, int32_t T, int32_t C, int32_t dtype, const void *x, const float *mu0,
+                                          const float *mu1, const void *gout0, const void *gout1, void *gx, float *gmu0,
+                                          float *gmu1, void *workspace, size_t workspace_bytes, void *stream);
+
+/*
+ * The five data-dependent mixes with their low-rank products inside (rwkv6_model.py:128-146), bf16, rank 32:
+ *   out[j] = x + (shift(x) - x) * l_j,   l_j = bias[j] + h_j wb[j]
+ * x, out[j], gout[j], gx dense [B,T,C]; h [B*T, 160] (the five tanh(x_mix A_j) side by side); wb [5,32,C]; bias [5,C];
+ * out / gout are host arrays of five device pointers.  Backward: gx, and gl [5, B*T, C] = the gradient of the l_j (the caller's
+ * products turn it into the gradients of h, wb and bias); gx holds the part that does not go through h.
+ * C a multiple of 8; pointers 16-byte aligned.
+ */
+WKV6_API int wkv6_lora_mix_forward(int32_t B, int32_t T, int32_t C, const void *x, const void *h, const void *wb,
+                                   const void *bias, void *const *out, void *stream);
+WKV6_API int wkv6_lora_mix_backward(int32_t B, int32_t T, int32_t C, const void *x, const void *h, const void *wb,
+                                    const void *bias, const void *const *gout, void *gx, void *gl, void *stream);
+
 /*
  * Activations of the channel-mix block over whole sequences, one launch per direction (n elements of `dtype`, dense,
  * pointers 16-byte aligned):

@@ -25,7 +25,8 @@ SYMBOLS = (
     "wkv6_split_segments", "wkv6_split_state_bytes", "wkv6_split_workspace_bytes", "wkv6_forward_split", "wkv6_backward_split",
     "wkv6_groupnorm_gate_forward", "wkv6_groupnorm_gate_backward", "wkv6_groupnorm_gate_workspace_bytes",
     "wkv6_groupnorm_silu_gate_forward", "wkv6_groupnorm_silu_gate_backward",
-    "wkv6_shift_mix_forward", "wkv6_shift_mix_backward", "wkv6_shift_mix_workspace_bytes", "wkv6_copy_2d_async",
+    "wkv6_shift_mix_forward", "wkv6_shift_mix_backward", "wkv6_shift_mix_workspace_bytes", "wkv6_shift_mix_pair_forward", "wkv6_shift_mix_pair_backward",
+    "wkv6_lora_mix_forward", "wkv6_lora_mix_backward", "wkv6_copy_2d_async",
     "wkv6_relu_sq_forward", "wkv6_relu_sq_backward", "wkv6_sigmoid_mul_forward", "wkv6_sigmoid_mul_backward",
     "wkv6_xla_forward", "wkv6_xla_backward", "wkv6_xla_forward_with_state", "wkv6_xla_forward_ckpt", "wkv6_xla_backward_ws",
     "wkv6_xla_buffer_bytes", "wkv6_xla_descriptor", "wkv6_xla_target",
@@ -130,6 +131,15 @@ def _load():
     lib.wkv6_shift_mix_backward.argtypes = [i32] * 6 + [vp] * 6 + [sz, vp]
     lib.wkv6_shift_mix_workspace_bytes.restype = sz
     lib.wkv6_shift_mix_workspace_bytes.argtypes = [i32] * 4
+    lib.wkv6_shift_mix_pair_forward.restype = ctypes.c_int
+    lib.wkv6_shift_mix_pair_forward.argtypes = [i32] * 4 + [vp] * 6
+    lib.wkv6_shift_mix_pair_backward.restype = ctypes.c_int
+    lib.wkv6_shift_mix_pair_backward.argtypes = [i32] * 4 + [vp] * 9 + [sz, vp]
+    vpp = ctypes.POINTER(vp)
+    lib.wkv6_lora_mix_forward.restype = ctypes.c_int
+    lib.wkv6_lora_mix_forward.argtypes = [i32] * 3 + [vp] * 4 + [vpp, vp]
+    lib.wkv6_lora_mix_backward.restype = ctypes.c_int
+    lib.wkv6_lora_mix_backward.argtypes = [i32] * 3 + [vp] * 4 + [vpp] + [vp] * 3
     for name, nptr in (("wkv6_relu_sq_forward", 2), ("wkv6_relu_sq_backward", 3), ("wkv6_sigmoid_mul_forward", 3),
                        ("wkv6_sigmoid_mul_backward", 5)):
         fn = getattr(lib, name)

@@ -17,7 +17,7 @@ from .channel_mix_ops import relu_sq, sigmoid_mul
 from .group_norm import GroupNormGate
 from .group_norm import groupnorm_gate_forward_raw
 from .ops import wkv6, wkv6_decode, wkv6_with_state
-from .time_mix_inputs import TimeMixInputs, shift_mix_vector
+from .time_mix_inputs import TimeMixInputs, shift_mix_pair
 
 
 _SIDE_STREAMS = {}
@@ -79,7 +79,7 @@ class TimeMix(nn.Module):
             self.w_b.bias.uniform_(-6.0, -1.0)  # decays exp(-exp(w)) spread between slow and fast channels
 
     def forward(self, x):
-        xr, xk, xv, xw, xg = self.mix_inputs(x)
+        xr, xk, xv, xw, xg = self.mix_inputs.split(x)
         r, k, v = self.dense_r(xr), self.dense_k(xk), self.dense_v(xv)
         w = self.w_b(torch.tanh(self.w_a(xw)))
         y = wkv6(r, k, v, w, self.time_faaaa, self.head_size)
@@ -93,7 +93,7 @@ class TimeMix(nn.Module):
     @torch.no_grad()
     def prefill(self, x):
         """Forward over a whole prompt; returns the output and the layer state (last input token, WKV state)."""
-        r, k, v, w, g = self._project(*self.mix_inputs(x))
+        r, k, v, w, g = self._project(*self.mix_inputs.split(x))
         y, S = wkv6_with_state(r, k, v, w, self.time_faaaa, self.head_size)
         gn = self.group_norm
         return self.dense_o(groupnorm_gate_forward_raw(y, g.contiguous(), gn.scale, gn.offset, gn.epsilon)), (x[:, -1:].clone(), S)
@@ -165,8 +165,7 @@ class ChannelMix(nn.Module):
         self.dense_receptance = nn.Linear(hidden_size, hidden_size, bias=False)
 
     def forward(self, x):
-        xk = shift_mix_vector(x, self.time_mix_k)
-        xr = shift_mix_vector(x, self.time_mix_r)
+        xk, xr = shift_mix_pair(x, self.time_mix_k, self.time_mix_r)
         k = relu_sq(self.dense_key(xk))                                   # one kernel per direction instead of relu, pow
         return sigmoid_mul(self.dense_receptance(xr), self.dense_value(k))   # ... and of sigmoid, mul
 

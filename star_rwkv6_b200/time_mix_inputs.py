@@ -6,8 +6,9 @@ projections (TimeMix.call, rwkv6_model.py:128-146):
     l_i     = tanh(x_mix A_i) B_i + b_i                 (DecomposerDense, rwkv6_model.py:11-24), i in r, k, v, w, g
     x_i     = x + x_shift * l_i
 
-The two interpolation steps are the fused kernels behind ``wkv6_shift_mix_forward / _backward`` (x is read once, no
-shifted copy is materialised); the two small matrix products are plain library GEMMs (torch.matmul / baddbmm).
+The interpolation steps are fused kernels (x is read once, no shifted copy is materialised).  For bf16 with the usual rank
+of 32 the products with B_i run inside the second one (``wkv6_lora_mix_forward / _backward``), so that the l_i exist in
+registers only; otherwise they are a batched library product in front of ``wkv6_shift_mix_forward / _backward``.
 """
 from __future__ import annotations
 
@@ -74,6 +75,86 @@ class _ShiftMixTensors(torch.autograd.Function):
         return _shift_mix_bwd(x, m, gout.to(x.dtype).contiguous(), False)
 
 
+class _ShiftMixPair(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, mu0, mu1):
+        _check_cuda(x, mu0, mu1)
+        x = x.contiguous()
+        mu = [m.detach().to(torch.float32).contiguous() for m in (mu0, mu1)]
+        ctx.save_for_backward(x, *mu)
+        ctx.mu_dtypes = mu0.dtype, mu1.dtype
+        B, T, C = x.shape
+        out = [torch.empty_like(x) for _ in range(2)]
+        with torch.cuda.device(x.device):
+            check(lib.wkv6_shift_mix_pair_forward(B, T, C, _DT[x.dtype], _ptr(x), _ptr(mu[0]), _ptr(mu[1]), _ptr(out[0]), _ptr(out[1]),
+                                                  _stream(x.device)))
+        return tuple(out)
+
+    @staticmethod
+    def backward(ctx, g0, g1):
+        x, mu0, mu1 = ctx.saved_tensors
+        B, T, C = x.shape
+        g0, g1 = g0.to(x.dtype).contiguous(), g1.to(x.dtype).contiguous()
+        gx = torch.empty_like(x)
+        gmu = [torch.empty((C,), dtype=torch.float32, device=x.device) for _ in range(2)]
+        nbytes = lib.wkv6_shift_mix_workspace_bytes(B, T, C, 2)
+        ws = torch.empty((nbytes,), dtype=torch.uint8, device=x.device) if nbytes else None
+        with torch.cuda.device(x.device):
+            check(lib.wkv6_shift_mix_pair_backward(B, T, C, _DT[x.dtype], _ptr(x), _ptr(mu0), _ptr(mu1), _ptr(g0), _ptr(g1), _ptr(gx),
+                                                   _ptr(gmu[0]), _ptr(gmu[1]), _ptr(ws), nbytes, _stream(x.device)))
+        return gx, gmu[0].to(ctx.mu_dtypes[0]), gmu[1].to(ctx.mu_dtypes[1])
+
+
+def _pointers(ts):
+    return (ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
+
+
+def _lora_mix_fwd(x, h, wb, bias, out):
+    B, T, C = x.shape
+    with torch.cuda.device(x.device):
+        check(lib.wkv6_lora_mix_forward(B, T, C, _ptr(x), _ptr(h), _ptr(wb), _ptr(bias), _pointers(out), _stream(x.device)))
+
+
+class _LoraMix(torch.autograd.Function):
+    """The five x + (shift(x) - x) * (bias_j + h_j wb_j) for x [B,T,C], h [B*T, 160], wb [5, 32, C], bias [5, 1, C], all bf16:
+    five tensors, or one [5, B, T, C] (``stacked``)."""
+
+    @staticmethod
+    def forward(ctx, x, h, wb, bias, stacked):
+        x, h, wb, bias = (t.contiguous() for t in (x, h, wb, bias))
+        ctx.save_for_backward(x, h, wb, bias)
+        ctx.stacked = stacked
+        out = torch.empty((5, *x.shape), dtype=x.dtype, device=x.device) if stacked else [torch.empty_like(x) for _ in range(5)]
+        _lora_mix_fwd(x, h, wb, bias, out)
+        return out if stacked else tuple(out)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, *gout):
+        x, h, wb, bias = ctx.saved_tensors
+        B, T, C = x.shape
+        gout = [g.contiguous() for g in (gout[0] if ctx.stacked else gout)]
+        gx = torch.empty_like(x)
+        gl = torch.empty((5, B * T, C), dtype=x.dtype, device=x.device)
+        with torch.cuda.device(x.device):
+            check(lib.wkv6_lora_mix_backward(B, T, C, _ptr(x), _ptr(h), _ptr(wb), _ptr(bias), _pointers(gout), _ptr(gx), _ptr(gl),
+                                             _stream(x.device)))
+        h5 = h.view(B * T, 5, -1).permute(1, 2, 0)                                              # [5, 32, B*T]
+        gh = torch.bmm(gl, wb.transpose(1, 2)).transpose(0, 1).reshape(h.shape)
+        return gx, gh, torch.bmm(h5, gl), gl.sum(1, keepdim=True), None
+
+
+def _lora_fits(x, h, wb, bias):
+    return (x.is_cuda and x.dim() == 3 and x.numel() > 0 and x.shape[-1] % 8 == 0 and wb.shape == (5, 32, x.shape[-1])
+            and all(t.dtype == torch.bfloat16 for t in (x, h, wb, bias))
+            and all(t.data_ptr() % 16 == 0 for t in (x, h, wb, bias)))
+
+
+def shift_mix_pair(x, mu0, mu1):
+    """(x + (shift(x) - x) * mu0, the same with mu1) for x [B,T,C] and two mixing vectors [C]: x is read once and gets one gradient."""
+    return _ShiftMixPair.apply(x, mu0, mu1)
+
+
 def shift_mix_vector(x, mu):
     """x + (shift(x) - x) * mu for x [B,T,C] and one mixing vector mu [C]."""
     return _ShiftMixVec.apply(x, mu)
@@ -99,9 +180,20 @@ class TimeMixInputs(torch.nn.Module):
         self.bias_b = torch.nn.Parameter(torch.zeros(5, 1, D))                 # dense_b biases (use_bias=True)
 
     def forward(self, x):
+        """[5, B, T, D]: xr, xk, xv, xw, xg stacked."""
+        return self._mixes(x, True)
+
+    def split(self, x):
+        """The same as five tensors (their gradients need not be stacked again on the way back)."""
+        return self._mixes(x, False)
+
+    def _mixes(self, x, stacked):
         B, T, D = x.shape
         x_mix = shift_mix_vector(x, self.time_mix_x)
         h = torch.tanh(x_mix.reshape(B * T, D) @ self.dense_a.to(x.dtype))                      # [B*T, 5R]
+        wb, bias = self.dense_b.to(x.dtype), self.bias_b.to(x.dtype)
+        if _lora_fits(x, h, wb, bias):
+            return _LoraMix.apply(x, h, wb, bias, stacked)
         h = h.reshape(B * T, 5, self.decomposer_size).transpose(0, 1)                            # [5, B*T, R]
-        l = torch.baddbmm(self.bias_b.to(x.dtype), h, self.dense_b.to(x.dtype))                  # [5, B*T, D]
+        l = torch.baddbmm(bias, h, wb)                                                           # [5, B*T, D]
         return shift_mix_tensors(x, l.reshape(5, B, T, D))                                       # xr, xk, xv, xw, xg
