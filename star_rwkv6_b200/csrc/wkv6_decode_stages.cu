@@ -21,19 +21,16 @@
 
 namespace wkv6 {
 
-constexpr int kStageThreads = 256;
-constexpr int kStageMaxPer = 32;  // channels per thread of the row kernel: D <= 8192
+constexpr int kStageThreads = 512;
+constexpr int kStageMaxPer = 16;  // channels per thread of the row kernel: D <= 8192
 
-__device__ __forceinline__ float block_sum_256(float x, float *scratch) {
+// every call of a kernel uses a scratch of its own
+__device__ __forceinline__ float block_sum(float x, float *scratch) {
     x = warp_sum(x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();  // scratch may still be read from a previous call
     if (lane == 0) scratch[warp] = x;
     __syncthreads();
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < kStageThreads / 32; ++i) t += scratch[i];
-    return t;
+    return warp_sum(lane < kStageThreads / 32 ? scratch[lane] : 0.f);
 }
 
 template <typename T> struct Pair;
@@ -61,27 +58,35 @@ template <> struct Pair<__half> {
     static __device__ __forceinline__ float round(float x) { return __half2float(__float2half_rn(x)); }
 };
 
-// One CTA per batch row; a thread owns pairs of neighbouring channels (pair index tid + 256 j).  xa_out / xs_out / mix1
-// may be NULL.  D even, D <= 8192.
-template <typename T>
+// One CTA per batch row; a thread owns kPairs pairs of neighbouring channels (pair index tid + 512 j).  xa_out / xs_out / mix1
+// may be NULL.  D even, D <= 1024 kPairs.  A few rows leave the chip idle, so the time is one chain: load, two block sums,
+// store.  Everything is requested at the start, the parameters too (read behind the sums by 256 threads with 16 predicated
+// pairs each it took 8.6 us at 16 x 4096).
+template <typename T, int kPairs>
 __global__ void __launch_bounds__(kStageThreads) decode_ln_shift_mix_kernel(int D, const void *x, const void *ln_w,
                                                                           const void *ln_b, float eps, void *prev,
                                                                           const float *mu0, const float *mu1, void *xa_out,
                                                                           void *xs_out, void *mix0, void *mix1) {
-    __shared__ float scratch[kStageThreads / 32];
-    constexpr int kPairs = kStageMaxPer / 2;
+    __shared__ float scratch[2][kStageThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
     const int npairs = D / 2;
-    float2 v[kPairs], pv[kPairs];
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 v[kPairs], pv[kPairs], lw[kPairs], lb[kPairs], m0[kPairs], m1[kPairs];
     float s = 0.f;
 #pragma unroll
     for (int j = 0; j < kPairs; ++j) {
         const int i = threadIdx.x + j * kStageThreads;
-        v[j] = i < npairs ? Pair<T>::load(x, row + 2 * i) : make_float2(0.f, 0.f);
-        pv[j] = i < npairs ? Pair<T>::load(prev, row + 2 * i) : make_float2(0.f, 0.f);
-        s += v[j].x + v[j].y;
+        const bool ok = i < npairs;
+        v[j] = ok ? Pair<T>::load(x, row + 2 * i) : zero;
+        pv[j] = ok ? Pair<T>::load(prev, row + 2 * i) : zero;
+        lw[j] = ok ? Pair<T>::load(ln_w, 2 * i) : zero;
+        lb[j] = ok ? Pair<T>::load(ln_b, 2 * i) : zero;
+        m0[j] = ok ? *reinterpret_cast<const float2 *>(mu0 + 2 * i) : zero;
+        m1[j] = ok && mix1 ? *reinterpret_cast<const float2 *>(mu1 + 2 * i) : zero;
     }
-    const float mean = block_sum_256(s, scratch) / D;
+#pragma unroll
+    for (int j = 0; j < kPairs; ++j) s += v[j].x + v[j].y;
+    const float mean = block_sum(s, scratch[0]) / D;
     float q = 0.f;
 #pragma unroll
     for (int j = 0; j < kPairs; ++j) {
@@ -91,26 +96,21 @@ __global__ void __launch_bounds__(kStageThreads) decode_ln_shift_mix_kernel(int 
             q += cx * cx + cy * cy;
         }
     }
-    const float rstd = rsqrtf(block_sum_256(q, scratch) / D + eps);
+    const float rstd = rsqrtf(block_sum(q, scratch[1]) / D + eps);
 #pragma unroll
     for (int j = 0; j < kPairs; ++j) {
         const int i = threadIdx.x + j * kStageThreads;
         if (i < npairs) {
-            const float2 lw = Pair<T>::load(ln_w, 2 * i), lb = Pair<T>::load(ln_b, 2 * i);
-            const float2 m0 = *reinterpret_cast<const float2 *>(mu0 + 2 * i);
             // the normalised value is rounded to the activation dtype first, as a separate LayerNorm would leave it
-            const float2 xa = make_float2(Pair<T>::round((v[j].x - mean) * rstd * lw.x + lb.x),
-                                          Pair<T>::round((v[j].y - mean) * rstd * lw.y + lb.y));
+            const float2 xa = make_float2(Pair<T>::round((v[j].x - mean) * rstd * lw[j].x + lb[j].x),
+                                          Pair<T>::round((v[j].y - mean) * rstd * lw[j].y + lb[j].y));
             const float2 xs = make_float2(pv[j].x - xa.x, pv[j].y - xa.y);
             const size_t o = row + 2 * i;
             Pair<T>::store(prev, o, xa);
             if (xa_out) Pair<T>::store(xa_out, o, xa);
             if (xs_out) Pair<T>::store(xs_out, o, xs);
-            Pair<T>::store(mix0, o, make_float2(fmaf(xs.x, m0.x, xa.x), fmaf(xs.y, m0.y, xa.y)));
-            if (mix1) {
-                const float2 m1 = *reinterpret_cast<const float2 *>(mu1 + 2 * i);
-                Pair<T>::store(mix1, o, make_float2(fmaf(xs.x, m1.x, xa.x), fmaf(xs.y, m1.y, xa.y)));
-            }
+            Pair<T>::store(mix0, o, make_float2(fmaf(xs.x, m0[j].x, xa.x), fmaf(xs.y, m0[j].y, xa.y)));
+            if (mix1) Pair<T>::store(mix1, o, make_float2(fmaf(xs.x, m1[j].x, xa.x), fmaf(xs.y, m1[j].y, xa.y)));
         }
     }
 }
@@ -121,12 +121,19 @@ struct Perm5 { int v[5]; };
 // batch rows, so that the R weight rows it needs are independent loads the compiler keeps in flight together.
 // h [B, 5R] (the x_mix A product, before tanh), wb [5, R, D], bias [5, D], xa / xs [B, D], out [5, B, D]; D even.
 // The result of mix m is written to out[perm.v[m]].
+// kR: R where it is the usual 32 (all weight rows are then requested before the tanh is staged: 11.4 -> 5 us at 16 x 4096), else 0.
 constexpr int kLoraRows = 4;
-template <typename T>
+template <typename T, int kR>
 __global__ void __launch_bounds__(128) decode_lora_mix_kernel(int B, int D, int R, const void *h, const void *wb,
                                                               const void *bias, const void *xa, const void *xs, void *out,
                                                               Perm5 perm) {
     extern __shared__ float sh[];  // [kLoraRows][R] tanh(h) of this mix
+    const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    float2 w[kR > 0 ? kR : 1];
+    if (kR > 0 && d < D) {
+#pragma unroll
+        for (int j = 0; j < kR; ++j) w[j] = Pair<T>::load(wb, ((size_t)blockIdx.z * kR + j) * D + d);
+    }
     const int m = blockIdx.z, b0 = blockIdx.y * kLoraRows, nb = min(kLoraRows, B - b0);
     for (int i = threadIdx.x; i < kLoraRows * R; i += blockDim.x) {
         const int rb = i / R, j = i - rb * R;
@@ -135,21 +142,25 @@ __global__ void __launch_bounds__(128) decode_lora_mix_kernel(int B, int D, int 
                         : 0.f;
     }
     __syncthreads();
-    const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (d >= D) return;
     float2 acc[kLoraRows];
 #pragma unroll
     for (int rb = 0; rb < kLoraRows; ++rb) acc[rb] = make_float2(0.f, 0.f);
     const size_t wbase = (size_t)m * R * D + d;
-#pragma unroll 8
-    for (int j = 0; j < R; ++j) {
-        const float2 wgt = Pair<T>::load(wb, wbase + (size_t)j * D);
+    auto step = [&](int j, float2 wgt) {
 #pragma unroll
         for (int rb = 0; rb < kLoraRows; ++rb) {
             const float hv = sh[rb * R + j];
             acc[rb].x = fmaf(hv, wgt.x, acc[rb].x);
             acc[rb].y = fmaf(hv, wgt.y, acc[rb].y);
         }
+    };
+    if (kR > 0) {
+#pragma unroll
+        for (int j = 0; j < (kR > 0 ? kR : 1); ++j) step(j, w[j]);
+    } else {
+#pragma unroll 8
+        for (int j = 0; j < R; ++j) step(j, Pair<T>::load(wb, wbase + (size_t)j * D));
     }
     const float2 bm = Pair<T>::load(bias, (size_t)m * D + d);
 #pragma unroll
@@ -212,12 +223,16 @@ int wkv6_decode_ln_shift_mix(int32_t B, int32_t D, int32_t dtype, float eps, con
     if (!pair_aligned(dtype, {x, ln_w, ln_b, prev, xa_out, xs_out, mix0, mix1}) || !pair_aligned(WKV6_F32, {mu0, mu1}))
         return fail(WKV6_ERR_INVALID, "wkv6_decode_ln_shift_mix: a pointer is not aligned to two elements");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == WKV6_F32)
-        decode_ln_shift_mix_kernel<float><<<B, kStageThreads, 0, st>>>(D, x, ln_w, ln_b, eps, prev, mu0, mu1, xa_out, xs_out, mix0, mix1);
-    else if (dtype == WKV6_BF16)
-        decode_ln_shift_mix_kernel<__nv_bfloat16><<<B, kStageThreads, 0, st>>>(D, x, ln_w, ln_b, eps, prev, mu0, mu1, xa_out, xs_out, mix0, mix1);
-    else
-        decode_ln_shift_mix_kernel<__half><<<B, kStageThreads, 0, st>>>(D, x, ln_w, ln_b, eps, prev, mu0, mu1, xa_out, xs_out, mix0, mix1);
+#define LN_SHIFT(T)                                                                                                                  \
+    do {                                                                                                                             \
+        auto kernel = D <= 2048 ? decode_ln_shift_mix_kernel<T, 2> : D <= 4096 ? decode_ln_shift_mix_kernel<T, 4>                     \
+                                                                               : decode_ln_shift_mix_kernel<T, kStageMaxPer / 2>;     \
+        kernel<<<B, kStageThreads, 0, st>>>(D, x, ln_w, ln_b, eps, prev, mu0, mu1, xa_out, xs_out, mix0, mix1);                       \
+    } while (0)
+    if (dtype == WKV6_F32) LN_SHIFT(float);
+    else if (dtype == WKV6_BF16) LN_SHIFT(__nv_bfloat16);
+    else LN_SHIFT(__half);
+#undef LN_SHIFT
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "decode_ln_shift_mix_kernel launch");
 }
@@ -242,9 +257,11 @@ int wkv6_decode_lora_mix(int32_t B, int32_t D, int32_t R, int32_t dtype, const v
     const dim3 grid((D / 2 + 127) / 128, (B + kLoraRows - 1) / kLoraRows, 5);
     const size_t smem = kLoraRows * R * sizeof(float);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == WKV6_F32) decode_lora_mix_kernel<float><<<grid, 128, smem, st>>>(B, D, R, h, wb, bias, xa, xs, out, pm);
-    else if (dtype == WKV6_BF16) decode_lora_mix_kernel<__nv_bfloat16><<<grid, 128, smem, st>>>(B, D, R, h, wb, bias, xa, xs, out, pm);
-    else decode_lora_mix_kernel<__half><<<grid, 128, smem, st>>>(B, D, R, h, wb, bias, xa, xs, out, pm);
+#define LORA(T) (R == 32 ? decode_lora_mix_kernel<T, 32> : decode_lora_mix_kernel<T, 0>)<<<grid, 128, smem, st>>>(B, D, R, h, wb, bias, xa, xs, out, pm)
+    if (dtype == WKV6_F32) LORA(float);
+    else if (dtype == WKV6_BF16) LORA(__nv_bfloat16);
+    else LORA(__half);
+#undef LORA
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "decode_lora_mix_kernel launch");
 }
