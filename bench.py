@@ -346,8 +346,6 @@ def run_b200(a):
     resolved = pkg.ops.resolve_variant(devs[0]["r"], u, N, variant)
     vname = {1: "seq", 2: "chunk"}[resolved]
     launches_per_step = {"seq": 4, "chunk": 3}[vname]  # chunk: forward, fast backward, general backward (exits at once when nothing is flagged)
-    if vname == "chunk" and pkg.ops.cut_along_T(devs[0]["r"], u, N, variant):
-        launches_per_step += 3  # a summary in front of either direction, the gu rows of the segments added up
     segmented = a.segments > 1 or (a.tshard and world > 1)
     collective = a.tshard and world > 1
     if segmented:

@@ -92,18 +92,6 @@ def resolve_variant(r, u, head_size: int, variant: int = _lib.VARIANT_AUTO) -> i
     return rc
 
 
-def _chunk_segments(p) -> int:
-    """Segments the library cuts this problem's sequences into on the chunked variant (1: not cut)."""
-    if lib.wkv6_resolve_variant(ctypes.byref(p)) != _lib.VARIANT_CHUNK:
-        return 1
-    return max(1, lib.wkv6_split_segments(ctypes.byref(p)))
-
-
-def cut_along_T(r, u, head_size: int, variant: int = _lib.VARIANT_AUTO) -> bool:
-    """Whether forward_raw / backward_raw cut these sequences into segments."""
-    return _chunk_segments(make_problem(r, u, head_size, out_dtype(r.dtype), variant)) > 1
-
-
 def forward_raw(r, k, v, w, u, head_size: int, *, s_in=None, s_map=None, want_state=False, want_ckpt=False,
                 variant: int = _lib.VARIANT_AUTO):
     """Launch the forward.  Returns (y, s_out or None, ckpt or None)."""
@@ -137,12 +125,6 @@ def forward_raw(r, k, v, w, u, head_size: int, *, s_in=None, s_map=None, want_st
             s_out.copy_(s_in.index_select(0, idx))
         return y, s_out, ckpt
     with torch.cuda.device(r.device):
-        if B * T * C > 0 and _chunk_segments(p) > 1:
-            nws = lib.wkv6_split_workspace_bytes(ctypes.byref(p), 0)
-            ws = torch.empty((nws,), dtype=torch.uint8, device=r.device)
-            check(lib.wkv6_forward_split(ctypes.byref(p), _ptr(r), _ptr(k), _ptr(v), _ptr(w), _ptr(u), _ptr(y), _ptr(s_in),
-                                         _ptr(s_map), kinds, _ptr(s_out), _ptr(ckpt), _ptr(ws), nws, _stream(r.device)))
-            return y, s_out, ckpt
         check(lib.wkv6_forward(ctypes.byref(p), _ptr(r), _ptr(k), _ptr(v), _ptr(w), _ptr(u), _ptr(y), _ptr(s_in),
                                _ptr(s_map), kinds, _ptr(s_out), _ptr(ckpt), _stream(r.device)))
     return y, s_out, ckpt
@@ -163,16 +145,6 @@ def backward_raw(r, k, v, w, u, gy, head_size: int, *, ckpt=None, variant: int =
     p = make_problem(r, u, head_size, ydt, variant)
     gr, gk, gv, gw = (_out_like(r, ydt) for _ in range(4))
     gu = torch.empty((B, H, N), dtype=torch.float32, device=r.device)
-    G = _chunk_segments(p) if ckpt is not None and B * T * C > 0 else 1
-    if G > 1:    # the gu rows of the segments come back separately
-        nbytes = lib.wkv6_split_workspace_bytes(ctypes.byref(p), 1)
-        ws = torch.empty((nbytes,), dtype=torch.uint8, device=r.device)
-        rows = torch.empty((G, B, H, N), dtype=torch.float32, device=r.device)
-        with torch.cuda.device(r.device):
-            check(lib.wkv6_backward_split(ctypes.byref(p), _ptr(r), _ptr(k), _ptr(v), _ptr(w), _ptr(u), _ptr(gy), _ptr(gr), _ptr(gk),
-                                          _ptr(gv), _ptr(gw), _ptr(rows), _ptr(ckpt), _ptr(ws), nbytes, _stream(r.device)))
-            check(lib.wkv6_sum_rows(_ptr(rows), G, gu.numel(), _ptr(gu), _stream(r.device)))
-        return gr, gk, gv, gw, gu
     nbytes = lib.wkv6_backward_workspace_bytes(ctypes.byref(p), 1 if ckpt is not None else 0)
     ws = torch.empty((nbytes,), dtype=torch.uint8, device=r.device) if nbytes else None
     with torch.cuda.device(r.device):
