@@ -339,6 +339,21 @@ WKV6_API int wkv6_lora_mix_backward(int32_t B, int32_t T, int32_t C, const void 
                                     const void *bias, const void *const *gout, void *gx, void *gl, void *stream);
 
 /*
+ * LayerNorm over the channels of `rows` tokens of D channels (a multiple of 8, at most 8192), bf16, with the residual addition
+ * in front of it (the norms of a block, rwkv6_model.py:197-215):
+ *   s = x + o (o may be NULL: s = x, s_out unused),   y = LayerNorm(s; gamma, beta, eps)
+ * stat (optional) receives mean and 1 / standard deviation, fp32 [rows][2], for the backward:
+ *   gx = gs + the gradient of s through the norm (gs, the gradient that reaches s past the norm, may be NULL); ggamma, gbeta.
+ * All pointers 16-byte aligned.
+ */
+WKV6_API int wkv6_layer_norm_forward(int64_t rows, int32_t D, float eps, const void *x, const void *o, const void *gamma,
+                                     const void *beta, void *s_out, void *y, float *stat, void *stream);
+WKV6_API size_t wkv6_layer_norm_workspace_bytes(int64_t rows, int32_t D);
+WKV6_API int wkv6_layer_norm_backward(int64_t rows, int32_t D, const void *s, const float *stat, const void *gamma,
+                                      const void *gy, const void *gs, void *gx, void *ggamma, void *gbeta, void *workspace,
+                                      size_t workspace_bytes, void *stream);
+
+/*
  * Activations of the channel-mix block over whole sequences, one launch per direction (n elements of `dtype`, dense,
  * pointers 16-byte aligned):
  *   wkv6_relu_sq_forward:      out = max(x, 0)^2          wkv6_relu_sq_backward:      gx = gout * 2 max(x, 0)

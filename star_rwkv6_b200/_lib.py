@@ -26,7 +26,8 @@ SYMBOLS = (
     "wkv6_groupnorm_gate_forward", "wkv6_groupnorm_gate_backward", "wkv6_groupnorm_gate_workspace_bytes",
     "wkv6_groupnorm_silu_gate_forward", "wkv6_groupnorm_silu_gate_backward",
     "wkv6_shift_mix_forward", "wkv6_shift_mix_backward", "wkv6_shift_mix_workspace_bytes", "wkv6_shift_mix_pair_forward", "wkv6_shift_mix_pair_backward",
-    "wkv6_lora_mix_forward", "wkv6_lora_mix_backward", "wkv6_copy_2d_async",
+    "wkv6_lora_mix_forward", "wkv6_lora_mix_backward",
+    "wkv6_layer_norm_forward", "wkv6_layer_norm_backward", "wkv6_layer_norm_workspace_bytes", "wkv6_copy_2d_async",
     "wkv6_relu_sq_forward", "wkv6_relu_sq_backward", "wkv6_sigmoid_mul_forward", "wkv6_sigmoid_mul_backward",
     "wkv6_xla_forward", "wkv6_xla_backward", "wkv6_xla_forward_with_state", "wkv6_xla_forward_ckpt", "wkv6_xla_backward_ws",
     "wkv6_xla_buffer_bytes", "wkv6_xla_descriptor", "wkv6_xla_target",
@@ -135,6 +136,12 @@ def _load():
     lib.wkv6_shift_mix_pair_forward.argtypes = [i32] * 4 + [vp] * 6
     lib.wkv6_shift_mix_pair_backward.restype = ctypes.c_int
     lib.wkv6_shift_mix_pair_backward.argtypes = [i32] * 4 + [vp] * 9 + [sz, vp]
+    lib.wkv6_layer_norm_forward.restype = ctypes.c_int
+    lib.wkv6_layer_norm_forward.argtypes = [i64, i32, ctypes.c_float] + [vp] * 8
+    lib.wkv6_layer_norm_workspace_bytes.restype = sz
+    lib.wkv6_layer_norm_workspace_bytes.argtypes = [i64, i32]
+    lib.wkv6_layer_norm_backward.restype = ctypes.c_int
+    lib.wkv6_layer_norm_backward.argtypes = [i64, i32] + [vp] * 9 + [sz, vp]
     vpp = ctypes.POINTER(vp)
     lib.wkv6_lora_mix_forward.restype = ctypes.c_int
     lib.wkv6_lora_mix_forward.argtypes = [i32] * 3 + [vp] * 4 + [vpp, vp]

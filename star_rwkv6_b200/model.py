@@ -3,8 +3,8 @@ model (rwkv6_model.py): EmbeddingLayer (:219-239), RWKV_Block (:197-215: x + Tim
 TimeMix (:116-196), ChannelMix (:48-83), OutputLayer (:240-259), RWKV6 (:260-276).
 
 Hand-written kernels: the WKV recurrence (``ops.wkv6``), the token-shift interpolations in front of the projections
-(``time_mix_inputs``) and the per-head GroupNorm + gate behind it (``group_norm``).  The dense projections, layer norms,
-embedding and loss are library calls (cuBLAS / ATen).  Used by ``bench.py --workload train_step`` and
+(``time_mix_inputs``), the per-head GroupNorm + gate behind it (``group_norm``) and the layer norms with the residual
+additions in front of them (``layer_norm``).  The dense projections and the embedding are library calls (cuBLAS / ATen).  Used by ``bench.py --workload train_step`` and
 ``tests/test_gpu_model.py``; weights are random (no checkpoint can be loaded here).
 """
 from __future__ import annotations
@@ -16,6 +16,7 @@ from . import decode_stages as ds
 from .channel_mix_ops import relu_sq, sigmoid_mul
 from .group_norm import GroupNormGate
 from .group_norm import groupnorm_gate_forward_raw
+from .layer_norm import layer_norm, residual_layer_norm
 from .ops import wkv6, wkv6_decode, wkv6_with_state
 from .time_mix_inputs import TimeMixInputs, shift_mix_pair
 
@@ -93,10 +94,13 @@ class TimeMix(nn.Module):
     @torch.no_grad()
     def prefill(self, x):
         """Forward over a whole prompt; returns the output and the layer state (last input token, WKV state)."""
-        r, k, v, w, g = self._project(*self.mix_inputs.split(x))
+        xr, xk, xv, xw, xg = self.mix_inputs.split(x)
+        r, k, v = self.dense_r(xr), self.dense_k(xk), self.dense_v(xv)
+        w = self.w_b(torch.tanh(self.w_a(xw)))
         y, S = wkv6_with_state(r, k, v, w, self.time_faaaa, self.head_size)
         gn = self.group_norm
-        return self.dense_o(groupnorm_gate_forward_raw(y, g.contiguous(), gn.scale, gn.offset, gn.epsilon)), (x[:, -1:].clone(), S)
+        z = groupnorm_gate_forward_raw(y, self.dense_g(xg), gn.scale, gn.offset, gn.epsilon, gate_is_raw=True)
+        return self.dense_o(z), (x[:, -1:].clone(), S)
 
     @torch.no_grad()
     def decode(self, x, state):
@@ -206,14 +210,15 @@ class Block(nn.Module):
         self.channel_mix = ChannelMix(hidden_size, expand_size)
 
     def forward(self, x):
-        x = x + self.time_mix(self.layer_norm_att(x))
-        return x + self.channel_mix(self.layer_norm_ffn(x))
+        x, h = residual_layer_norm(x, None, self.layer_norm_att)
+        x, h = residual_layer_norm(x, self.time_mix(h), self.layer_norm_ffn)
+        return x + self.channel_mix(h)
 
     @torch.no_grad()
     def prefill(self, x):
-        o, st_att = self.time_mix.prefill(self.layer_norm_att(x))
-        x = x + o
-        o, st_ffn = self.channel_mix.prefill(self.layer_norm_ffn(x))
+        o, st_att = self.time_mix.prefill(layer_norm(x, self.layer_norm_att))
+        x, h = residual_layer_norm(x, o, self.layer_norm_ffn)
+        o, st_ffn = self.channel_mix.prefill(h)
         return x + o, (st_att, st_ffn)
 
     @torch.no_grad()
@@ -243,34 +248,34 @@ class RWKV6(nn.Module):
     def forward(self, tokens, checkpoint_blocks: bool = False):
         """``checkpoint_blocks``: keep only each block's input for the backward and recompute the block there (a
         24-layer, 2048-wide model at 32 k tokens per step would otherwise hold about 6 GB of activations per block)."""
-        x = self.embedding_ln(self.embedding(tokens))
+        x = layer_norm(self.embedding(tokens), self.embedding_ln)
         for blk in self.blocks:
             if checkpoint_blocks and torch.is_grad_enabled():
                 from torch.utils.checkpoint import checkpoint
                 x = checkpoint(blk, x, use_reentrant=False)
             else:
                 x = blk(x)
-        return self.output_layer(self.output_ln(x))
+        return self.output_layer(layer_norm(x, self.output_ln))
 
     @torch.no_grad()
     def prefill(self, tokens):
         """Prompt pass: logits of the last position [B,1,V] and the per-layer states for ``decode``."""
-        x = self.embedding_ln(self.embedding(tokens))
+        x = layer_norm(self.embedding(tokens), self.embedding_ln)
         states = []
         for blk in self.blocks:
             x, st = blk.prefill(x)
             states.append(st)
-        return self.output_layer(self.output_ln(x[:, -1:])), states
+        return self.output_layer(layer_norm(x[:, -1:], self.output_ln)), states
 
     @torch.no_grad()
     def decode(self, token, states, fused: bool = True):
         """One new token per sequence ([B,1] ids); ``states`` is updated in place (CUDA-graph friendly).  ``fused``:
         the element-wise stages of every block run as this package's decode-stage kernels (15 launches per block
         instead of about 40 framework operations); False keeps the plain framework operations."""
-        x = self.embedding_ln(self.embedding(token))
+        x = layer_norm(self.embedding(token), self.embedding_ln)
         for blk, st in zip(self.blocks, states):
             x = blk.decode(x, st, fused)
-        return self.output_layer(self.output_ln(x))
+        return self.output_layer(layer_norm(x, self.output_ln))
 
     def to_bf16_(self):
         """bf16 weights for the projections and norms; the small fp32 operands of the kernels (u, GroupNorm scale and

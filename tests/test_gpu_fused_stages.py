@@ -1,6 +1,6 @@
-"""Fused stages of the model's blocks against float64 evaluations of the same expressions: the pair of vector mixes and the five
-data-dependent mixes with their low-rank products, forward and backward, at sizes around their tiles (channel groups of
-32 / 128 / 256, tiles of 16 rows, runs of 4 and 8 tokens, batch boundaries)."""
+"""Fused stages of the model's blocks against float64 evaluations of the same expressions: the pair of vector mixes, the five
+data-dependent mixes with their low-rank products, and the layer norm with the residual addition, forward and backward, at
+sizes around their tiles (channel groups of 32 / 128 / 256, tiles of 16 rows, runs of 4 rows and 8 tokens, batch boundaries)."""
 import pytest
 import torch
 
@@ -54,3 +54,32 @@ def test_low_rank_mixes(B, T, C, stacked):
     ref = torch.autograd.grad(out64, a64, go.double())
     for a, b in zip((out if stacked else torch.stack(out), *got), (out64, *ref)):
         assert _err(a, b) <= 2 * TOL          # gl is rounded to bf16 before the products that make gh, gwb and gbias
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (5, 768), (33, 1032), (9, 2056), (700, 2048), (6, 4104), (3, 8192)])
+@pytest.mark.parametrize("add,use_sum", [(False, False), (True, True), (True, False), (False, True)])
+def test_layer_norm(rows, D, add, use_sum):
+    from star_rwkv6_b200.layer_norm import _fits, residual_layer_norm
+    g = torch.Generator(device="cuda").manual_seed(D)
+    ln = torch.nn.LayerNorm(D, eps=1e-5).cuda().bfloat16()
+    with torch.no_grad():
+        ln.weight.copy_(_randn(g, D) + 1); ln.bias.copy_(_randn(g, D))
+    x = (_randn(g, rows, D) + 3).requires_grad_(True)       # a mean well away from zero
+    o = _randn(g, rows, D).requires_grad_(True) if add else None
+    assert _fits(x, ln)
+    gy, gs = _randn(g, rows, D), _randn(g, rows, D)
+    s, y = residual_layer_norm(x, o, ln)
+    ins = [x] + ([o] if add else []) + [ln.weight, ln.bias]
+    got = torch.autograd.grad([y] + ([s] if use_sum else []), ins, [gy] + ([gs] if use_sum else []))
+    i64 = [t.detach().double().requires_grad_(True) for t in ins]
+    total = i64[0] + i64[1] if add else i64[0]
+    if add:
+        total = total + (s.detach().double() - total.detach())       # the sum as it is stored, rounded
+    y64 = torch.nn.functional.layer_norm(total, (D,), i64[-2], i64[-1], 1e-5)
+    ref = torch.autograd.grad([y64] + ([total] if use_sum else []), i64, [gy.double()] + ([gs.double()] if use_sum else []))
+    assert _err(y, y64) <= TOL and _err(s, total) <= TOL
+    for a, b in zip(got, ref):
+        assert _err(a, b) <= TOL
+    with torch.no_grad():
+        s1, y1 = residual_layer_norm(x, o, ln)
+    assert torch.equal(y1, y) and torch.equal(s1, s)
