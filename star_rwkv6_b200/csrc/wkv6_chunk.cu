@@ -27,9 +27,9 @@ int sm_count() {
 
 // Launch with programmatic stream serialization: the kernel's CTAs may become resident while the kernel before it in the
 // stream drains.  A kernel launched this way calls ptx::grid_dependency_wait() before its first access to global
-// memory, so whatever ran before it has completed by then.  Used for the general backward behind the fast one (its
-// launch, which normally finds every flag at zero, then costs 1.5 us instead of 4.5); chaining the other kernels of a
-// split step the same way measured no gain.
+// memory that depends on it, so whatever ran before it has completed by then.  Used for the general backward behind the fast
+// one (its launch, which normally finds every flag at zero, then costs 1.5 us instead of 4.5) and for the main kernels of a cut
+// call behind the summaries.
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_behind(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
                                  Args &&...args) {
@@ -194,20 +194,21 @@ static int launch_forward(const wkv6_problem *p, const Dims &d, const SegGeom &s
     if ((rc = make_map(&mv, v, p, d, "v"))) return rc;
     if ((rc = make_map(&mw, w, p, d, "w"))) return rc;
     if ((rc = make_map(&my, y ? y : r, p, d, "y"))) return rc;  // y == NULL: states only, the map is never used
-    ChunkFwdArgs a{};
+    ChunkCutArgs a{};
     a.u = u; a.u_dtype = p->u_dtype; a.s_in = s_in; a.s_map = s_map; a.s_kinds = s_kinds; a.s_dtype = p->s_dtype;
     a.s_out = s_out; a.write_y = (y != nullptr); a.ckpt = static_cast<__nv_bfloat16 *>(ckpt);
     a.reverse_state = false; a.dec_out = nullptr; a.B = p->B; a.T = p->T; a.H = p->H;
     a.seg = seg; a.fold_b = fold.b; a.fold_dec = fold.dec; a.fold_sub = fold.sub;
     a.skip_load_chunk = g_skip_load_chunk.load() + 1;
-    cudaError_t e = cudaFuncSetAttribute(chunk_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         ChunkFwdSmem::kAlloc);
+    const bool cut = fold.b != nullptr;
+    const void *kernel = cut ? reinterpret_cast<const void *>(chunk_fwd_kernel<true>) : reinterpret_cast<const void *>(chunk_fwd_kernel<false>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ChunkFwdSmem::kAlloc);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(chunk_fwd_kernel)");
     const unsigned grid = (unsigned)(seg.G * p->B * p->H);
-    if (fold.b != nullptr) {
-        e = launch_behind(chunk_fwd_kernel, grid, 256, ChunkFwdSmem::kAlloc, st, mr, mk, mv, mw, my, a);
+    if (cut) {
+        e = launch_behind(chunk_fwd_kernel<true>, grid, 256, ChunkFwdSmem::kAlloc, st, mr, mk, mv, mw, my, a);
     } else {
-        chunk_fwd_kernel<<<grid, 256, ChunkFwdSmem::kAlloc, st>>>(mr, mk, mv, mw, my, a);
+        chunk_fwd_kernel<false><<<grid, 256, ChunkFwdSmem::kAlloc, st>>>(mr, mk, mv, mw, my, a);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "chunk_fwd_kernel launch");
@@ -326,7 +327,7 @@ static int launch_summary(const wkv6_problem *p, const Dims &d, const SegGeom &s
     if ((rc = make_map(&m1, x1, p, d, "x1"))) return rc;
     if ((rc = make_map(&m2, x2, p, d, "x2"))) return rc;
     if ((rc = make_map(&mw, w, p, d, "w"))) return rc;
-    ChunkFwdArgs a{};
+    ChunkCutArgs a{};
     a.u = nullptr; a.u_dtype = WKV6_F32; a.s_dtype = WKV6_F32; a.s_out = b_out; a.B = p->B; a.T = p->T; a.H = p->H;
     a.write_y = false; a.reverse_state = reverse; a.dec_out = dec_log2_out;
     a.skip_mod = skip_mod; a.skip_rem = skip_rem; a.seg = seg;

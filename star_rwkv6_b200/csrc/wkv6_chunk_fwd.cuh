@@ -29,6 +29,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "sm100_ptx.cuh"
 #include "wkv6_seq.cuh"
 
@@ -157,9 +159,6 @@ __device__ __forceinline__ void fold_segments(float (&S)[16], const float *bsum,
 struct ChunkFwdArgs {
     const void *u; int u_dtype;
     const void *s_in; const int64_t *s_map; int s_kinds; int s_dtype; void *s_out;
-    SegGeom seg;
-    const float *fold_b, *fold_dec;  // summaries of the pieces before this segment ([pieces][B*H]); NULL: one segment
-    int fold_sub;                    // pieces per segment
     __nv_bfloat16 *ckpt;  // optional [B*H][T/64][64*64] bf16 chunk-start states in operand (swizzled) layout
     int B, T, H;
     bool write_y;         // false: only states / checkpoints are produced
@@ -171,6 +170,12 @@ struct ChunkFwdArgs {
     // Test hook (wkv6_debug_inject): the forward never requests the input tiles of chunk index skip_load_chunk - 1
     // (0 = off), so the wait for them runs out with no copy outstanding and the kernel takes its error path.
     int skip_load_chunk;
+};
+
+struct ChunkCutArgs : ChunkFwdArgs {   // of launches over segments
+    SegGeom seg;
+    const float *fold_b, *fold_dec;  // summaries of the pieces before this segment ([pieces][B*H]); NULL: one segment
+    int fold_sub;                    // pieces per segment
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -219,12 +224,15 @@ __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
     return *reinterpret_cast<uint32_t *>(&h);
 }
 
+// CUT: the launch covers segments (SegGeom); otherwise whole sequences, whose loop then carries no segment offsets (1024
+// sequences of 64 chunks: 702 against 712 us with one kernel for both; the longer argument struct alone cost that much).
+template <bool CUT>
 __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_r,
                                                            const __grid_constant__ CUtensorMap tm_k,
                                                            const __grid_constant__ CUtensorMap tm_v,
                                                            const __grid_constant__ CUtensorMap tm_w,
                                                            const __grid_constant__ CUtensorMap tm_y,
-                                                           const ChunkFwdArgs a) {
+                                                           const std::conditional_t<CUT, ChunkCutArgs, ChunkFwdArgs> a) {
     using namespace ptx;
     using SM = ChunkFwdSmem;
     // Declared with the alignment the swizzled tiles need, so that the compiler keeps every access in the shared
@@ -252,9 +260,12 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     const int w4 = warp & 3, half = warp >> 2, n0 = 4 * half;
     const int q = lane & 3, r0 = lane >> 2;
     const int ta = 16 * w4 + r0;
-    const SegPlace pl = seg_place(a.seg, a.B, a.T, a.H);
-    const int b = pl.b, h = pl.h, c0 = pl.c0;
-    const int nchunks = pl.cend - c0;
+    SegPlace pl{};
+    if constexpr (CUT) pl = seg_place(a.seg, a.B, a.T, a.H);
+    const int total = (a.T + kChunk - 1) / kChunk, c0 = CUT ? pl.c0 : 0;
+    const unsigned seq = CUT ? (unsigned)pl.seq : blockIdx.x;
+    const int b = CUT ? pl.b : blockIdx.x / a.H, h = CUT ? pl.h : blockIdx.x % a.H;
+    const int nchunks = CUT ? pl.cend - c0 : total;
     WKV6_CSTAMP(0);
 
     if (tid == 0) {
@@ -328,7 +339,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
                 }
             }
         }
-        if (a.fold_b != nullptr && pl.g > 0) {
+        if constexpr (CUT) if (pl.g > 0) {
             // launched behind the summary kernel with programmatic serialization: nothing before this point reads what that
             // kernel writes or writes what it reads
             grid_dependency_wait();
@@ -365,7 +376,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     const bool copy_thread = (tid == 32);
     if (copy_thread) {
         if (a.ckpt != nullptr) {  // state at the start of the first chunk, already in operand layout
-            bulk_store(a.ckpt + ((size_t)pl.seq * pl.total + c0) * 4096, sSB, kTile);
+            bulk_store(a.ckpt + ((size_t)seq * total + c0) * 4096, sSB, kTile);
             bulk_commit();
         }
     }
@@ -675,7 +686,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
             // the state entering the next chunk is complete in shared memory: checkpoint it for the backward.
             // Its read is drained (bulk_wait_read) before the next chunk's first barrier, ahead of the rewrite.
             if (a.ckpt != nullptr && ic + 1 < nchunks) {
-                bulk_store(a.ckpt + ((size_t)pl.seq * pl.total + c + 1) * 4096, sSB, kTile);
+                bulk_store(a.ckpt + ((size_t)seq * total + c + 1) * 4096, sSB, kTile);
                 bulk_commit();
             }
         }
@@ -724,8 +735,8 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
         if (err != 0) atomicExch(&g_chunk_status, err);
         bulk_wait<0>();
     }
-    if (err == 0 && a.s_out != nullptr && pl.cend == pl.total) {
-        const size_t so2 = (size_t)pl.seq * 4096;
+    if (err == 0 && a.s_out != nullptr && (!CUT || pl.cend == total)) {
+        const size_t so2 = (size_t)seq * 4096;
 #pragma unroll
         for (int nn = 0; nn < 4; ++nn)
 #pragma unroll

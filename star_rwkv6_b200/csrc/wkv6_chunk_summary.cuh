@@ -30,7 +30,7 @@ struct ChunkSumSmem {
 __global__ void __launch_bounds__(256, 4) chunk_summary_kernel(const __grid_constant__ CUtensorMap tm_x1,
                                                                const __grid_constant__ CUtensorMap tm_x2,
                                                                const __grid_constant__ CUtensorMap tm_w,
-                                                               const ChunkFwdArgs a) {
+                                                               const ChunkCutArgs a) {
     using namespace ptx;
     using SM = ChunkSumSmem;
     extern __shared__ __align__(1024) uint8_t wkv6_chunk_smem[];
