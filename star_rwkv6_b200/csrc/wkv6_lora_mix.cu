@@ -6,15 +6,19 @@
 // As separate steps (bias broadcast into the result, batched product onto it, element-wise kernel) the five l tensors crossed
 // HBM four times and the broadcast ran at 1 TB/s (about 300 us forward at 4004 x 4096 in all).  Here l lives in accumulators only; what is
 // left is x in and five results out (12 bytes per token and channel), backward x and five gradients in, gx and five gradients out
-// (24).  Measured at 4004 x 4096: forward 66 us (3 TB/s; L1 at 87 %, mostly the weight fragments each tile re-reads), at 4096 x 2048
-// 42 us forward and 65 us backward.
+// (24).  Measured with a cold L2 at 4004 x 4096: forward 73 us, backward 150 us (forward L1 at 87 %, mostly the weight fragments each
+// tile re-reads); at 4096 x 2048 49 us and 83 us.
 //
 // A product over k = 32 is two mma.m16n8k16 steps: the tensor work is a tenth of the transfer time, so the warp-level
 // instruction is enough, and its fragments can be arranged so that nothing is staged:
 //   * column n of the four n8 tiles j of a 32-channel group stands for channel 8 (n / 2) + 2 j + n % 2, so that the accumulators
 //     of a thread are eight neighbouring channels (16-byte accesses to x, gout and the results);
-//   * reduction index (step s, register half hh, quad lane q, element e) stands for k = 8 q + 4 s + 2 hh + e, so that a thread's
-//     share of a row of h_j is one 16-byte load.
+//   * reduction index (step s, register half hh, quad lane q, element e) stands for k = 16 s + 4 q + 2 hh + e, so that a thread's
+//     share of a row of h_j is one 8-byte load per step.
+// l has the bits of the general path (the library's batched product with the bias added onto it, then shift_mix_*_kernel): each
+// step sums the same 16 k, and product and sum are rounded where that path stores them.  The gradients of a training step are not
+// determined to better than that: behind a token whose WKV output is nearly zero the per-head norm magnifies single rounding
+// steps of bf16, so that 8 elements of l in a million one step off (another order of the k) move gradients by percents.
 // One CTA: 128 channels, B_j in shared memory in fragment order (40 KB), eight warps = four groups of 32 channels x two runs
 // of rows.  A warp walks tiles of 16 rows; the backward walks down, because gx[t] needs sum_j gout_j l_j of token t + 1.
 #include <cuda_bf16.h>
@@ -27,6 +31,7 @@ namespace wkv6 {
 constexpr int kMixes = 5, kRank = 32, kMixCols = 128, kMixThreads = 256, kMixLanes = 2;  // kMixLanes: runs of rows per CTA
 constexpr int kMixWords = kMixes * 4 * 4 * 32 * 4;                                       // [mix][group][tile][lane][step, half]
 constexpr int kMixSmem = kMixWords * 4 + kMixes * kMixCols * 4;
+constexpr int kMixBwdSmem = kMixSmem + kMixes * 2 * kMixThreads * 16;                     // and a tile's l, [mix][row half][thread]
 
 struct MixOut { __nv_bfloat16 *p[5]; };
 struct MixGrad { const __nv_bfloat16 *p[5]; };
@@ -42,6 +47,13 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// a lane's share of a row of h_j: k = 4 q .. 4 q + 3 and 16 + 4 q .. 16 + 4 q + 3 (p points at its first element)
+__device__ __forceinline__ uint4 ld_h(const __nv_bfloat16 *p, bool ok) {
+    const uint2 zero = make_uint2(0u, 0u);
+    const uint2 a = ok ? __ldg(reinterpret_cast<const uint2 *>(p)) : zero, b = ok ? __ldg(reinterpret_cast<const uint2 *>(p + 16)) : zero;
+    return make_uint4(a.x, a.y, b.x, b.y);
 }
 
 __device__ __forceinline__ uint4 ld_row(const __nv_bfloat16 *p, bool ok) {
@@ -90,7 +102,7 @@ __device__ __forceinline__ void stage_weights(const __nv_bfloat16 *wb, const __n
     for (int e = 0; e < kEach; ++e) {
         const int i = threadIdx.x + e * kMixThreads, cp = i % (kMixCols / 2), kp = i / (kMixCols / 2) % (kRank / 2), m = i / (kMixCols / 2 * (kRank / 2));
         const int c = 2 * cp, k = 2 * kp, grp = c >> 5, cc = c & 31, n = 2 * (cc >> 3), tile = (cc & 7) >> 1;
-        const int q = k >> 3, w = 2 * ((k >> 2) & 1) + ((k >> 1) & 1);
+        const int q = (k >> 2) & 3, w = 2 * (k >> 4) + ((k >> 1) & 1);
         uint32_t *d = sB + ((((m * 4 + grp) * 4 + tile) * 32) + 4 * n + q) * 4 + w;
         d[0] = __byte_perm(lo[e], hi[e], 0x5410);    // channel c:     n
         d[16] = __byte_perm(lo[e], hi[e], 0x7632);   // channel c + 1: n + 1, four lanes further
@@ -101,6 +113,12 @@ __device__ __forceinline__ void stage_weights(const __nv_bfloat16 *wb, const __n
     __syncthreads();
 }
 
+// product rounded, then the sum with the bias rounded, as the general path leaves them
+__device__ __forceinline__ float2 biased(float x, float y, float2 bias) {
+    const float2 p = __bfloat1622float2(__floats2bfloat162_rn(x, y));
+    return __bfloat1622float2(__floats2bfloat162_rn(p.x + bias.x, p.y + bias.y));
+}
+
 // l of one mix for this thread's two rows (g, g + 8) and eight channels
 __device__ __forceinline__ void mix_product(const uint4 &ha, const uint4 &hb, const uint32_t *sB, const float *sBias, float (&la)[8], float (&lb)[8]) {
     const uint32_t a0[4] = {ha.x, hb.x, ha.y, hb.y}, a1[4] = {ha.z, hb.z, ha.w, hb.w};
@@ -108,12 +126,10 @@ __device__ __forceinline__ void mix_product(const uint4 &ha, const uint4 &hb, co
     for (int j = 0; j < 4; ++j) {
         const uint4 b = *reinterpret_cast<const uint4 *>(sB + j * 128);
         const float2 bi = *reinterpret_cast<const float2 *>(sBias + 2 * j);
-        float d[4] = {bi.x, bi.y, bi.x, bi.y};
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
         mma_16816(d, a0, b.x, b.y);
         mma_16816(d, a1, b.z, b.w);
-        // rounded as the separate product would leave it: the gradients of r, k and u are differences of nearly equal terms, and
-        // with l in fp32 they moved by 6 % against a model whose other products are rounded (either way about float64)
-        const float2 a = __bfloat1622float2(__floats2bfloat162_rn(d[0], d[1])), c = __bfloat1622float2(__floats2bfloat162_rn(d[2], d[3]));
+        const float2 a = biased(d[0], d[1], bi), c = biased(d[2], d[3], bi);
         la[2 * j] = a.x; la[2 * j + 1] = a.y;
         lb[2 * j] = c.x; lb[2 * j + 1] = c.y;
     }
@@ -138,8 +154,8 @@ __global__ void __launch_bounds__(kMixThreads, 2) lora_mix_fwd_kernel(LoraGeom G
     uint4 ha[kMixes], hb[kMixes], xa4, xb4, pa4, pb4;
     auto fetch_h = [&](int t, int m) {
         const int ra = 16 * t + g, rb = ra + 8;
-        ha[m] = ld_row(h + (size_t)ra * (kMixes * kRank) + m * kRank + 8 * q, ra < G.rows);
-        hb[m] = ld_row(h + (size_t)rb * (kMixes * kRank) + m * kRank + 8 * q, rb < G.rows);
+        ha[m] = ld_h(h + (size_t)ra * (kMixes * kRank) + m * kRank + 4 * q, ra < G.rows);
+        hb[m] = ld_h(h + (size_t)rb * (kMixes * kRank) + m * kRank + 4 * q, rb < G.rows);
     };
     auto fetch_x = [&](int t) {
         const int ra = 16 * t + g, rb = ra + 8;
@@ -177,7 +193,9 @@ __global__ void __launch_bounds__(kMixThreads, 2) lora_mix_fwd_kernel(LoraGeom G
 
 // gl_j[t] = gout_j[t] (x[t-1] - x[t]);  gx[t] = sum_j gout_j[t] (1 - l_j[t]) + s[t+1],  s[t] = sum_j gout_j[t] l_j[t]
 // (s[t+1] = 0 at the last token of a batch row).  Inside a tile s[t+1] comes from the lane four further (the second rows for
-// the last of the first eight), across tiles it is carried; a run starts with the s of the row behind it.
+// the last of the first eight), across tiles it is carried; a run starts with the s of the row behind it.  gx is summed in the
+// order of shift_mix_bwd_kernel, s[t+1] first and then mix by mix, so that it has that kernel's bits: each thread keeps its l in
+// shared memory until the s of the tile are known (4096 x 2048: 83 us; 71 us with s[t+1] added last, 87 us with l kept in registers).
 __global__ void __launch_bounds__(kMixThreads) lora_mix_bwd_kernel(LoraGeom G, const __nv_bfloat16 *__restrict__ x,
                                                                    const __nv_bfloat16 *__restrict__ h,
                                                                    const __nv_bfloat16 *__restrict__ wb,
@@ -196,16 +214,21 @@ __global__ void __launch_bounds__(kMixThreads) lora_mix_bwd_kernel(LoraGeom G, c
     const size_t plane = (size_t)G.rows * G.C;
     const uint32_t *myB = sB + (grp * 4 * 32 + lane) * 4;
     const float *myBias = sBias + 32 * grp + 8 * q;
+    uint4 *sL = reinterpret_cast<uint4 *>(sBias + kMixes * kMixCols) + threadIdx.x;
     float carry[8];   // lanes g = 0: s of the first row of the tile behind
 #pragma unroll
     for (int e = 0; e < 8; ++e) carry[e] = 0.f;
     // what the next tile reads is requested while this one is computed (see the forward)
     uint4 ha[kMixes], hb[kMixes], goa4[kMixes], gob4[kMixes], xa4, xb4, pa4, pb4;
-    auto fetch_mix = [&](int t, int m) {
+    auto fetch_h = [&](int t, int m) {
         const int ra = 16 * t + g, rb = ra + 8;
         const bool oka = ra < G.rows && (t != t1 || g == 0), okb = rb < G.rows && t != t1;
-        ha[m] = ld_row(h + (size_t)ra * (kMixes * kRank) + m * kRank + 8 * q, oka);
-        hb[m] = ld_row(h + (size_t)rb * (kMixes * kRank) + m * kRank + 8 * q, okb);
+        ha[m] = ld_h(h + (size_t)ra * (kMixes * kRank) + m * kRank + 4 * q, oka);
+        hb[m] = ld_h(h + (size_t)rb * (kMixes * kRank) + m * kRank + 4 * q, okb);
+    };
+    auto fetch_g = [&](int t, int m) {
+        const int ra = 16 * t + g, rb = ra + 8;
+        const bool oka = ra < G.rows && (t != t1 || g == 0), okb = rb < G.rows && t != t1;
         const __nv_bfloat16 *pg = gout.p[m] + (size_t)ra * G.C + ch;
         goa4[m] = ld_row(pg, oka && chan);
         gob4[m] = ld_row(pg + (size_t)8 * G.C, okb && chan);
@@ -220,7 +243,7 @@ __global__ void __launch_bounds__(kMixThreads) lora_mix_bwd_kernel(LoraGeom G, c
     const int first = t1 < G.tiles ? t1 : t1 - 1;
     fetch_x(first);
 #pragma unroll
-    for (int m = 0; m < kMixes; ++m) fetch_mix(first, m);
+    for (int m = 0; m < kMixes; ++m) { fetch_h(first, m); fetch_g(first, m); }
     for (int t = first; t >= t0; --t) {
         const bool ahead = t == t1, more = t > t0;    // ahead: only s of its first row is wanted
         const int ra = 16 * t + g, rb = ra + 8;
@@ -236,31 +259,40 @@ __global__ void __launch_bounds__(kMixThreads) lora_mix_bwd_kernel(LoraGeom G, c
         if (more) fetch_x(t - 1);
         float sa[8], sb[8], aa[8], ab[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sa[e] = sb[e] = aa[e] = ab[e] = 0.f;
+        for (int e = 0; e < 8; ++e) sa[e] = sb[e] = 0.f;
 #pragma unroll
         for (int m = 0; m < kMixes; ++m) {
             float la[8], lb[8], ga[8], gb[8];
             mix_product(ha[m], hb[m], myB + m * (4 * 4 * 128), myBias + m * kMixCols, la, lb);
             unpack8(goa4[m], ga); unpack8(gob4[m], gb);
-            if (more) fetch_mix(t - 1, m);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                sa[e] = fmaf(ga[e], la[e], sa[e]); sb[e] = fmaf(gb[e], lb[e], sb[e]);
-                aa[e] = fmaf(-ga[e], la[e], aa[e] + ga[e]); ab[e] = fmaf(-gb[e], lb[e], ab[e] + gb[e]);
-                ga[e] *= da[e]; gb[e] *= db[e];
-            }
-            __nv_bfloat16 *po = gl + m * plane + i;
-            if (oka) *reinterpret_cast<uint4 *>(po) = pack8(ga);
-            if (okb) *reinterpret_cast<uint4 *>(po + (size_t)8 * G.C) = pack8(gb);
+            for (int e = 0; e < 8; ++e) { sa[e] = fmaf(ga[e], la[e], sa[e]); sb[e] = fmaf(gb[e], lb[e], sb[e]); }
+            sL[(2 * m) * kMixThreads] = pack8(la); sL[(2 * m + 1) * kMixThreads] = pack8(lb);
+            if (more) fetch_h(t - 1, m);
         }
         const bool enda = (ra + 1) % G.T == 0, endb = (rb + 1) % G.T == 0;   // last token of a batch row: nothing comes back
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const float na = __shfl_sync(0xffffffffu, g == 0 ? sb[e] : sa[e], (lane + 4) & 31);
             const float nb = __shfl_sync(0xffffffffu, g == 0 ? carry[e] : sb[e], (lane + 4) & 31);
-            aa[e] += enda ? 0.f : na;
-            ab[e] += endb ? 0.f : nb;
+            aa[e] = enda ? 0.f : na;
+            ab[e] = endb ? 0.f : nb;
             carry[e] = sa[e];
+        }
+#pragma unroll
+        for (int m = 0; m < kMixes; ++m) {
+            float la[8], lb[8], ga[8], gb[8];
+            unpack8(sL[(2 * m) * kMixThreads], la); unpack8(sL[(2 * m + 1) * kMixThreads], lb);
+            unpack8(goa4[m], ga); unpack8(gob4[m], gb);
+            if (more) fetch_g(t - 1, m);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                aa[e] += fmaf(-ga[e], la[e], ga[e]); ab[e] += fmaf(-gb[e], lb[e], gb[e]);
+                ga[e] *= da[e]; gb[e] *= db[e];
+            }
+            __nv_bfloat16 *po = gl + m * plane + i;
+            if (oka) *reinterpret_cast<uint4 *>(po) = pack8(ga);
+            if (okb) *reinterpret_cast<uint4 *>(po + (size_t)8 * G.C) = pack8(gb);
         }
         if (oka) *reinterpret_cast<uint4 *>(gx + i) = pack8(aa);
         if (okb) *reinterpret_cast<uint4 *>(gx + i + (size_t)8 * G.C) = pack8(ab);
@@ -324,10 +356,12 @@ int wkv6_lora_mix_backward(int32_t B, int32_t T, int32_t C, const void *x, const
     dim3 grid;
     const LoraGeom G = lora_geom(B, T, C, 1, 4, &grid);
     using bf = __nv_bfloat16;
-    lora_mix_bwd_kernel<<<grid, kMixThreads, kMixSmem, static_cast<cudaStream_t>(stream)>>>(
+    cudaError_t e = cudaFuncSetAttribute(lora_mix_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixBwdSmem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(lora_mix_bwd_kernel)");
+    lora_mix_bwd_kernel<<<grid, kMixThreads, kMixBwdSmem, static_cast<cudaStream_t>(stream)>>>(
         G, static_cast<const bf *>(x), static_cast<const bf *>(h), static_cast<const bf *>(wb), static_cast<const bf *>(bias),
         go, static_cast<bf *>(gx), static_cast<bf *>(gl));
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "lora_mix_bwd_kernel launch");
 }
 
