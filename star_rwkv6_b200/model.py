@@ -169,7 +169,8 @@ class ChannelMix(nn.Module):
         self.dense_receptance = nn.Linear(hidden_size, hidden_size, bias=False)
 
     def forward(self, x):
-        xk, xr = shift_mix_pair(x, self.time_mix_k, self.time_mix_r)
+        # gradients with the bits of two mixes: those in front of this block follow single rounding steps of bf16
+        xk, xr = shift_mix_pair(x, self.time_mix_k, self.time_mix_r, separate_gx=True)
         k = relu_sq(self.dense_key(xk))                                   # one kernel per direction instead of relu, pow
         return sigmoid_mul(self.dense_receptance(xr), self.dense_value(k))   # ... and of sigmoid, mul
 

@@ -77,12 +77,12 @@ class _ShiftMixTensors(torch.autograd.Function):
 
 class _ShiftMixPair(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, mu0, mu1):
+    def forward(ctx, x, mu0, mu1, separate_gx):
         _check_cuda(x, mu0, mu1)
         x = x.contiguous()
         mu = [m.detach().to(torch.float32).contiguous() for m in (mu0, mu1)]
         ctx.save_for_backward(x, *mu)
-        ctx.mu_dtypes = mu0.dtype, mu1.dtype
+        ctx.mu_dtypes, ctx.separate_gx = (mu0.dtype, mu1.dtype), separate_gx
         B, T, C = x.shape
         out = [torch.empty_like(x) for _ in range(2)]
         with torch.cuda.device(x.device):
@@ -95,6 +95,9 @@ class _ShiftMixPair(torch.autograd.Function):
         x, mu0, mu1 = ctx.saved_tensors
         B, T, C = x.shape
         g0, g1 = g0.to(x.dtype).contiguous(), g1.to(x.dtype).contiguous()
+        if ctx.separate_gx:
+            (gx, gmu0), (gx1, gmu1) = _shift_mix_bwd(x, mu0, g0, True), _shift_mix_bwd(x, mu1, g1, True)
+            return gx.add_(gx1), gmu0.to(ctx.mu_dtypes[0]), gmu1.to(ctx.mu_dtypes[1]), None
         gx = torch.empty_like(x)
         gmu = [torch.empty((C,), dtype=torch.float32, device=x.device) for _ in range(2)]
         nbytes = lib.wkv6_shift_mix_workspace_bytes(B, T, C, 2)
@@ -102,7 +105,7 @@ class _ShiftMixPair(torch.autograd.Function):
         with torch.cuda.device(x.device):
             check(lib.wkv6_shift_mix_pair_backward(B, T, C, _DT[x.dtype], _ptr(x), _ptr(mu0), _ptr(mu1), _ptr(g0), _ptr(g1), _ptr(gx),
                                                    _ptr(gmu[0]), _ptr(gmu[1]), _ptr(ws), nbytes, _stream(x.device)))
-        return gx, gmu[0].to(ctx.mu_dtypes[0]), gmu[1].to(ctx.mu_dtypes[1])
+        return gx, gmu[0].to(ctx.mu_dtypes[0]), gmu[1].to(ctx.mu_dtypes[1]), None
 
 
 def _pointers(ts):
@@ -150,9 +153,11 @@ def _lora_fits(x, h, wb, bias):
             and all(t.data_ptr() % 16 == 0 for t in (x, h, wb, bias)))
 
 
-def shift_mix_pair(x, mu0, mu1):
-    """(x + (shift(x) - x) * mu0, the same with mu1) for x [B,T,C] and two mixing vectors [C]: x is read once and gets one gradient."""
-    return _ShiftMixPair.apply(x, mu0, mu1)
+def shift_mix_pair(x, mu0, mu1, separate_gx: bool = False):
+    """(x + (shift(x) - x) * mu0, the same with mu1) for x [B,T,C] and two mixing vectors [C]: x is read once and gets one gradient.
+    ``separate_gx``: that gradient with the bits of two ``shift_mix_vector`` calls, whose gradients are rounded before they are added
+    (one pass more, backward)."""
+    return _ShiftMixPair.apply(x, mu0, mu1, separate_gx)
 
 
 def shift_mix_vector(x, mu):

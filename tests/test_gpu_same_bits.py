@@ -30,3 +30,41 @@ def test_low_rank_mixes(B, T, C, stacked):
     ref = torch.autograd.grad(want, b, go)
     for x, y in zip((out if stacked else torch.stack(out), *got), (want, *ref)):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("B,T,C", [(1, 1, 8), (2, 31, 264), (3, 33, 64), (2, 1003, 768), (1, 65, 2048)])
+def test_pair_of_vector_mixes(B, T, C, dtype):
+    from star_rwkv6_b200.time_mix_inputs import shift_mix_pair, shift_mix_vector     # as ChannelMix calls it
+    g = torch.Generator(device="cuda").manual_seed(T + C)
+    x, go = _randn(g, B, T, C, dtype=dtype), [_randn(g, B, T, C, dtype=dtype) for _ in range(2)]
+    mu = [torch.rand(C, generator=g, device="cuda") for _ in range(2)]
+    a, b = _leaves([x, *mu]), _leaves([x, *mu])
+    out = shift_mix_pair(*a, separate_gx=True)
+    got = torch.autograd.grad(out, a, go)
+    want = [shift_mix_vector(b[0], m) for m in b[1:]]
+    ref = torch.autograd.grad(want, b, go)
+    for p, q in zip((*out, *got), (*want, *ref)):
+        assert torch.equal(p, q)
+
+
+def test_channel_mix_gradients():
+    """The channel-mix block against the same block with the two mixes as separate calls."""
+    from star_rwkv6_b200 import model
+    from star_rwkv6_b200.time_mix_inputs import shift_mix_vector
+    torch.manual_seed(0)
+    cm = model.ChannelMix(768, 1024).cuda()
+    for n, p in cm.named_parameters():
+        if p.dim() == 2:
+            p.data = p.data.bfloat16()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, go = _randn(g, 2, 203, 768), _randn(g, 2, 203, 768)
+    a, b = _leaves([x]), _leaves([x])
+    got = torch.autograd.grad(cm(a[0]), a + list(cm.parameters()), go)
+    pair, model.shift_mix_pair = model.shift_mix_pair, lambda x, m0, m1, **kw: (shift_mix_vector(x, m0), shift_mix_vector(x, m1))
+    try:
+        want = torch.autograd.grad(cm(b[0]), b + list(cm.parameters()), go)
+    finally:
+        model.shift_mix_pair = pair
+    for p, q in zip(got, want):
+        assert torch.equal(p, q)
