@@ -20,6 +20,22 @@ __device__ __forceinline__ float exp2f_fast(float x) {
     return y;
 }
 
+// exp(z - mx) of two logits.  The difference is formed before it is scaled: it is exact for logits near the maximum, where one
+// fused multiply-add z log2(e) - mx log2(e) is off by the rounding of its second term (3e-4 of the result at mx = 1e4), and no
+// term overflows for logits at the end of the type's range.  The packed instructions do both steps at the cost of that one.
+__device__ __forceinline__ float2 exp_pair(float2 z, float2 neg_mx) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    unsigned long long d, m, c;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(z.x), "f"(z.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(m) : "f"(neg_mx.x), "f"(neg_mx.y));
+    asm("mov.b64 %0, {%1, %1};" : "=l"(c) : "f"(kLog2e));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(m));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(c));
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
+    return make_float2(exp2f_fast(r.x), exp2f_fast(r.y));
+}
+
 constexpr int kXentThreads = 512;
 constexpr int kXentMaxVecs = 16;  // 16-byte vectors per thread: V <= 512 * 16 * 8 = 65536
 
@@ -52,7 +68,6 @@ template <int VECS>
 __global__ void __launch_bounds__(kXentThreads, VECS == 16 ? 1 : VECS == 4 ? 2 : 3)
 softmax_xent_kernel(int64_t rows, int V, __nv_bfloat16 *__restrict__ logits, const int64_t *__restrict__ targets, float scale,
                     float *__restrict__ loss) {
-    constexpr float kLog2e = 1.4426950408889634f;
     extern __shared__ uint4 next_row[];  // [VECS][kXentThreads]
     __shared__ float scratch[kXentThreads / 32];
     const int nvec = V >> 3, tid = threadIdx.x;
@@ -92,7 +107,7 @@ softmax_xent_kernel(int64_t rows, int V, __nv_bfloat16 *__restrict__ logits, con
             }
         }
         mx = xent_block_reduce(mx, true, scratch);
-        const float shift = -mx * kLog2e;
+        const float2 neg_mx = make_float2(-mx, -mx);
         float sum = 0.f;
 #pragma unroll
         for (int j = 0; j < VECS; ++j) {
@@ -100,14 +115,14 @@ softmax_xent_kernel(int64_t rows, int V, __nv_bfloat16 *__restrict__ logits, con
                 const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(&z[j]);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float2 f = __bfloat1622float2(p[e]);
-                    sum += exp2f_fast(fmaf(f.x, kLog2e, shift)) + exp2f_fast(fmaf(f.y, kLog2e, shift));
+                    const float2 x = exp_pair(__bfloat1622float2(p[e]), neg_mx);
+                    sum += x.x + x.y;
                 }
             }
         }
         sum = xent_block_reduce(sum, false, scratch);
         if (tid == 0) loss[row] = ignore ? 0.f : (mx + logf(sum)) - target_logit;
-        const float sc = ignore ? 0.f : scale, f0 = sc / sum;
+        const float sc = ignore ? 0.f : scale, inv = 1.f / sum;
         const int tvec = ignore ? -1 : (int)(tgt >> 3), telem = (int)(tgt & 7);
 #pragma unroll
         for (int j = 0; j < VECS; ++j) {
@@ -117,16 +132,16 @@ softmax_xent_kernel(int64_t rows, int V, __nv_bfloat16 *__restrict__ logits, con
                 float g[8];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float2 f = __bfloat1622float2(p[e]);
-                    g[2 * e] = exp2f_fast(fmaf(f.x, kLog2e, shift)) * f0;
-                    g[2 * e + 1] = exp2f_fast(fmaf(f.y, kLog2e, shift)) * f0;
+                    const float2 x = exp_pair(__bfloat1622float2(p[e]), neg_mx);
+                    g[2 * e] = x.x * inv;
+                    g[2 * e + 1] = x.y * inv;
                 }
                 if (i == tvec) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) g[e] -= e == telem ? sc : 0.f;
+                    for (int e = 0; e < 8; ++e) g[e] -= e == telem ? 1.f : 0.f;
                 }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(g[2 * e], g[2 * e + 1]);
+                for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(g[2 * e] * sc, g[2 * e + 1] * sc);
                 zrow[i] = z[j];
             }
         }

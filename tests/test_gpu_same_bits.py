@@ -68,3 +68,20 @@ def test_channel_mix_gradients():
         model.shift_mix_pair = pair
     for p, q in zip(got, want):
         assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("V", [8, 4104, 65536])
+def test_loss_of_logits_at_the_end_of_the_range(V):
+    """exp(z - max) is formed from the difference: no term overflows where the scaled logit would (|z| > 2.36e38), and the
+    probabilities of a row that is one value throughout are equal and sum to one."""
+    from star_rwkv6_b200.loss import lm_loss
+    logits = torch.zeros(3, V, device="cuda", dtype=torch.bfloat16)
+    logits[0, 3], logits[0, 5] = 3.2e38, -3.2e38
+    logits[1] = 3.2e38
+    logits[2] = -2.5e38
+    targets = torch.tensor([3, 1, 2], device="cuda")
+    z = logits.clone().requires_grad_(True)
+    lm_loss(z * 1, targets).backward()
+    p = torch.softmax(logits.double(), 1)
+    p[torch.arange(3), targets] -= 1
+    assert float((z.grad.double() - p / 3).abs().max()) <= 2 ** -8 / 3
