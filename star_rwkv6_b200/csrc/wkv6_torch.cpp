@@ -82,9 +82,10 @@ struct Call {
     int backward_G() const { return xt == at::kHalf ? 1 : G; }   // the backward of fp16 inputs is not split
 };
 
-// Fills the problem from the operator's five tensors; false when they are not what the native path handles.
+// Fills the problem from the operator's five tensors; false when they are not what the native path handles.  cut: the
+// library may cut the sequences into segments.
 bool make_call(const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u, int64_t N, int64_t variant,
-               Call &c) {
+               bool cut, Call &c) {
     if (r.dim() != 3 || N <= 0) return false;
     c.B = r.size(0); c.T = r.size(1); c.C = r.size(2);
     if (c.B == 0 || c.T == 0 || c.C == 0 || c.C % N != 0) return false;
@@ -109,7 +110,7 @@ bool make_call(const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &
     const int variant_of = api.resolve_variant(&p);
     if (variant_of < 0) return false;
     c.chunked = variant_of == WKV6_VARIANT_CHUNK;
-    c.G = api.split_segments(&p);
+    c.G = cut ? api.split_segments(&p) : 1;
     return true;
 }
 
@@ -141,9 +142,9 @@ void ok(int rc) { TORCH_CHECK(rc == 0, "wkv6_b200 error ", rc, ": ", api.last_er
 
 struct WKV6Function : public torch::autograd::Function<WKV6Function> {
     static Tensor forward(AutogradContext *ctx, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w,
-                          const Tensor &u, int64_t N, int64_t variant) {
+                          const Tensor &u, int64_t N, int64_t variant, bool cut) {
         Call c;
-        TORCH_CHECK(make_call(r, k, v, w, u, N, variant, c), "wkv6: unsupported call");   // checked by the caller
+        TORCH_CHECK(make_call(r, k, v, w, u, N, variant, cut, c), "wkv6: unsupported call");   // checked by the caller
         Tensor y = like(r, c.yt, c.dense);
         // what the backward needs beside the inputs: the chunk checkpoints, or the segments' entering states
         Tensor kept;
@@ -159,6 +160,7 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
         ctx->save_for_backward({r, k, v, w, u, kept});
         ctx->saved_data["N"] = N;
         ctx->saved_data["variant"] = variant;
+        ctx->saved_data["cut"] = cut;
         return y;
     }
 
@@ -171,7 +173,8 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
             at::NoGradGuard no_grad;
             c10::cuda::CUDAGuard guard(r.device());
             Call c;
-            TORCH_CHECK(make_call(r, k, v, w, u, ctx->saved_data["N"].toInt(), ctx->saved_data["variant"].toInt(), c),
+            TORCH_CHECK(make_call(r, k, v, w, u, ctx->saved_data["N"].toInt(), ctx->saved_data["variant"].toInt(),
+                                  ctx->saved_data["cut"].toBool(), c),
                         "wkv6: unsupported call");
             Tensor gy = grads[0];
             if (gy.strides() != r.strides() || reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 != 0)
@@ -210,7 +213,7 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
             for (auto &t : out) t = t.detach().requires_grad_(true);
             out = (*err)(std::move(out));
         }
-        out.resize(7);
+        out.resize(8);
         return out;
     }
 };
@@ -219,17 +222,18 @@ PyObject *none() { Py_RETURN_NONE; }
 
 #define ARG(i) THPVariable_Unpack(args[i])
 
-// wkv6(r, k, v, w, u, head_size, variant) -> y or None
+// wkv6(r, k, v, w, u, head_size, variant, cut = True) -> y or None
 PyObject *py_wkv6(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 7 || !plain_mode()) return none();
+    if ((n != 7 && n != 8) || !plain_mode()) return none();
     for (int i = 0; i < 5; ++i)
         if (!plain_tensor(args[i])) return none();
     const int64_t N = PyLong_AsLongLong(args[5]), variant = PyLong_AsLongLong(args[6]);
+    const bool cut = n < 8 || PyObject_IsTrue(args[7]) == 1;
     if (PyErr_Occurred()) return nullptr;
     const Tensor &r = ARG(0), &k = ARG(1), &v = ARG(2), &w = ARG(3), &u = ARG(4);
     Call c;
-    if (!make_call(r, k, v, w, u, N, variant, c)) return none();
+    if (!make_call(r, k, v, w, u, N, variant, cut, c)) return none();
     const bool grad = at::GradMode::is_enabled() && (r.requires_grad() || k.requires_grad() || v.requires_grad() ||
                                                      w.requires_grad() || u.requires_grad());
     Tensor y;
@@ -237,7 +241,7 @@ PyObject *py_wkv6(PyObject *, PyObject *const *args, Py_ssize_t n) {
         pybind11::gil_scoped_release no_gil;
         c10::cuda::CUDAGuard guard(r.device());
         if (grad) {
-            y = WKV6Function::apply(r, k, v, w, u, N, variant);
+            y = WKV6Function::apply(r, k, v, w, u, N, variant, cut);
         } else {
             y = like(r, c.yt, c.dense);
             if (run_forward(c, r, k, v, w, u, y, nullptr, 0, nullptr, nullptr) != 0)
@@ -249,17 +253,18 @@ PyObject *py_wkv6(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// with_state(r, k, v, w, u, init_state or None, head_size, variant) -> (y, state) or None
+// with_state(r, k, v, w, u, init_state or None, head_size, variant, cut = True) -> (y, state) or None
 PyObject *py_with_state(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 8 || !plain_mode()) return none();
+    if ((n != 8 && n != 9) || !plain_mode()) return none();
     for (int i = 0; i < 5; ++i)
         if (!plain_tensor(args[i])) return none();
     const int64_t N = PyLong_AsLongLong(args[6]), variant = PyLong_AsLongLong(args[7]);
+    const bool cut = n < 9 || PyObject_IsTrue(args[8]) == 1;
     if (PyErr_Occurred()) return nullptr;
     const Tensor &r = ARG(0), &k = ARG(1), &v = ARG(2), &w = ARG(3), &u = ARG(4);
     Call c;
-    if (!make_call(r, k, v, w, u, N, variant, c)) return none();
+    if (!make_call(r, k, v, w, u, N, variant, cut, c)) return none();
     const void *s_in = nullptr;
     int32_t kinds = 0;
     at::ScalarType st = at::kFloat;

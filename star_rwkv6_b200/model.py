@@ -83,7 +83,9 @@ class TimeMix(nn.Module):
         xr, xk, xv, xw, xg = self.mix_inputs.split(x)
         r, k, v = self.dense_r(xr), self.dense_k(xk), self.dense_v(xv)
         w = self.w_b(torch.tanh(self.w_a(xw)))
-        y = wkv6(r, k, v, w, self.time_faaaa, self.head_size)
+        # in one piece: the per-head norm behind it magnifies single rounding steps of y into percents of the gradients, so a row's
+        # gradients would depend on how its batch is cut
+        y = wkv6(r, k, v, w, self.time_faaaa, self.head_size, cut=False)
         return self.dense_o(self.group_norm(y, self.dense_g(xg), gate_is_raw=True))   # SiLU of the gate inside the kernel
 
     def _project(self, xr, xk, xv, xw, xg):

@@ -231,10 +231,13 @@ def _autograd_backward(ctx, gy, _g_ckpt):
 _forward_op.register_autograd(_autograd_backward, setup_context=_setup_context)
 
 
-def wkv6(r, k, v, w, u, head_size: int, variant: int = _lib.VARIANT_AUTO) -> torch.Tensor:
-    """Differentiable WKV6 with a zero initial state: y[B,T,C] from r,k,v,w [B,T,C] and u [H,N]."""
+def wkv6(r, k, v, w, u, head_size: int, variant: int = _lib.VARIANT_AUTO, cut: bool = True) -> torch.Tensor:
+    """Differentiable WKV6 with a zero initial state: y[B,T,C] from r,k,v,w [B,T,C] and u [H,N].
+
+    ``cut``: the library may cut sequences along T where B*H of them would leave SMs idle.  A row's last bits then depend on the
+    batch size it arrives in; False walks every sequence in one piece.  Compiled, traced and mode-wrapped calls are never cut."""
     if not torch.compiler.is_compiling():
-        y = _native.wkv6(r, k, v, w, u, head_size, variant)
+        y = _native.wkv6(r, k, v, w, u, head_size, variant, cut)
         if y is not None:
             return y
     need_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (r, k, v, w, u))
@@ -243,11 +246,11 @@ def wkv6(r, k, v, w, u, head_size: int, variant: int = _lib.VARIANT_AUTO) -> tor
 
 
 def wkv6_with_state(r, k, v, w, u, head_size: int, init_state=None, state_map=None,
-                    variant: int = _lib.VARIANT_AUTO):
+                    variant: int = _lib.VARIANT_AUTO, cut: bool = True):
     """Forward only, with an optional initial state and the final state returned (no autograd), as the
-    reference's with-state kernel (rwkv_kernel/jax_kernel/rwkv_kernels.cu:165-190)."""
+    reference's with-state kernel (rwkv_kernel/jax_kernel/rwkv_kernels.cu:165-190).  ``cut``: see ``wkv6``."""
     if state_map is None and not torch.compiler.is_compiling():
-        out = _native.with_state(r, k, v, w, u, init_state, head_size, variant)
+        out = _native.with_state(r, k, v, w, u, init_state, head_size, variant, cut)
         if out is not None:
             return out
     with torch.no_grad():

@@ -22,21 +22,25 @@ from .. import _lib, ops
 class RWKVKernelOperator:
     def __init__(self, head_size, max_sequence_length=None, variant="auto", segments=1):
         """``segments``: an integer G > 1 cuts every sequence into G pieces along T that run concurrently (bf16, head size
-        64); 1 and "auto" leave it to the library, which cuts where B*H sequences would leave SMs idle."""
+        64); 1 and "auto" leave it to the library, which cuts where B*H sequences would leave SMs idle (a row's last bits then
+        depend on the batch size it arrives in); "whole" walks every sequence in one piece.  Calls with a state take 1 for
+        an integer.  Compiled (torch.compile), traced and mode-wrapped calls are not cut by the library: they end in the
+        registered custom operator, so few long sequences are slower there and agree to rounding."""
         self.head_size = int(head_size)
         self.max_sequence_length = max_sequence_length
         self.variant = _lib.VARIANTS[variant] if isinstance(variant, str) else int(variant)
         self.segments = segments
 
     def __call__(self, r, k, v, w, u, return_state=False, init_state=None, state_map=None):
+        cut = self.segments != "whole"
         if state_map is None and not torch.compiler.is_compiling():
             # the plain calls without Python in between; None: not one of them, or arguments that need the checks below
             if return_state:
-                out = ops._native.with_state(r, k, v, w, u, init_state, self.head_size, self.variant)
+                out = ops._native.with_state(r, k, v, w, u, init_state, self.head_size, self.variant, cut)
                 if out is not None:
                     return out
-            elif init_state is None and self.segments in (1, "auto"):
-                y = ops._native.wkv6(r, k, v, w, u, self.head_size, self.variant)
+            elif init_state is None and self.segments in (1, "auto", "whole"):
+                y = ops._native.wkv6(r, k, v, w, u, self.head_size, self.variant, cut)
                 if y is not None:
                     return y, None
         B, T, C = r.shape
@@ -90,13 +94,13 @@ class RWKVKernelOperator:
                 with torch.no_grad():  # decode step: dedicated state-streaming kernel
                     return ops.wkv6_decode(r, k, v, w, u, self.head_size, state=init_state, state_map=state_map)
             return ops.wkv6_with_state(r, k, v, w, u, self.head_size, init_state=init_state, state_map=state_map,
-                                       variant=self.variant)
+                                       variant=self.variant, cut=cut)
         assert init_state is None and state_map is None, "init_state / state_map need return_state=True"
         G = self.segments
-        if G != 1 and r.dtype == torch.bfloat16 and self.head_size == 64 and self.variant != _lib.VARIANT_SEQ and r.is_contiguous():
+        if G not in (1, "whole") and r.dtype == torch.bfloat16 and self.head_size == 64 and self.variant != _lib.VARIANT_SEQ and r.is_contiguous():
             from .. import segments as seg
             if G == "auto":
                 G = seg.auto_segments(B, T, H)
             if G > 1 and T % G == 0:
                 return seg.wkv6_segmented(r, k, v, w, u, self.head_size, segments=G), None
-        return ops.wkv6(r, k, v, w, u, self.head_size, variant=self.variant), None
+        return ops.wkv6(r, k, v, w, u, self.head_size, variant=self.variant, cut=cut), None

@@ -85,3 +85,24 @@ def test_loss_of_logits_at_the_end_of_the_range(V):
     p = torch.softmax(logits.double(), 1)
     p[torch.arange(3), targets] -= 1
     assert float((z.grad.double() - p / 3).abs().max()) <= 2 ** -8 / 3
+
+
+def test_time_mix_walks_sequences_in_one_piece():
+    """A shape whose sequences the operator would cut: the block's gradients have the bits of the uncut call."""
+    from star_rwkv6_b200 import model
+    torch.manual_seed(0)
+    tm = model.TimeMix(128).cuda()
+    for n, p in tm.named_parameters():
+        if not n.endswith(("time_faaaa", "scale", "offset", "time_mix_x")):
+            p.data = p.data.bfloat16()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, go = _randn(g, 1, 300, 128), _randn(g, 1, 300, 128)
+    a, b = _leaves([x]), _leaves([x])
+    got = torch.autograd.grad(tm(a[0]), a + list(tm.parameters()), go)
+    wkv6, model.wkv6 = model.wkv6, lambda *t, **kw: torch.ops.wkv6_b200.forward(*t, True, 0)[0]
+    try:
+        want = torch.autograd.grad(tm(b[0]), b + list(tm.parameters()), go)
+    finally:
+        model.wkv6 = wkv6
+    for p, q in zip(got, want):
+        assert torch.equal(p, q)

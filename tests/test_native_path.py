@@ -1,5 +1,6 @@
-"""The native call path of the torch operator (csrc/wkv6_torch.cpp) against the registered custom ops on the same inputs:
-both end in the same kernels, so results are equal bit for bit."""
+"""The native call path of the torch operator (csrc/wkv6_torch.cpp) against the registered custom ops on the same inputs: where
+sequences are walked in one piece both end in the same kernels, so results are equal bit for bit.  Where the library cuts them (the
+custom ops never do) results agree to rounding."""
 import pytest
 import torch
 
@@ -52,3 +53,31 @@ def test_second_derivative_is_refused():
     (gr,) = torch.autograd.grad(ops.wkv6(*leaves, 64), leaves[:1], gy, create_graph=True)
     with pytest.raises(RuntimeError, match="not differentiable"):
         gr.sum().backward()
+
+
+def _gradients(call, x, u, gy):
+    leaves = [t.detach().requires_grad_(True) for t in (*x, u)]
+    y = call(*leaves)
+    return (y.detach(), *torch.autograd.grad(y, leaves, gy))
+
+
+@pytest.mark.parametrize("B,T,H,dtype,tol", [(1, 1003, 12, torch.bfloat16, 2e-2), (2, 300, 3, torch.float32, 2e-5)])
+def test_cut_and_whole_sequences(B, T, H, dtype, tol):
+    """A shape that the library cuts: in one piece on request, with the custom ops' bits; cut, with theirs to rounding (bf16: states
+    at the segments' ends from bf16 products; fp32: another order of a few hundred sums)."""
+    from star_rwkv6_b200 import _lib, ops
+    from star_rwkv6_b200.rwkv_kernel.torch_rwkv_kernel import RWKVKernelOperator
+    x, u, gy = _inputs(B, T, H, 64, dtype, 8)
+    gy = gy.to(dtype)
+    assert _lib.lib.wkv6_split_segments(ops.make_problem(x[0], u, 64, dtype, 0)) > 1
+    want = _gradients(lambda *a: torch.ops.wkv6_b200.forward(*a, 64, True, 0)[0], x, u, gy)
+    whole = _gradients(lambda *a: RWKVKernelOperator(64, T, segments="whole")(*a)[0], x, u, gy)
+    cut = _gradients(lambda *a: RWKVKernelOperator(64, T)(*a)[0], x, u, gy)
+    for name, a, b, c in zip(("y", "gr", "gk", "gv", "gw"), whole, cut, want):
+        assert torch.equal(a, c), name
+        assert float((b.double() - c.double()).norm() / c.double().norm()) <= tol, name
+    assert float((whole[5] - want[5]).abs().max()) <= B * 2 ** -24 * float(want[5].abs().max()) + 1e-12
+    s0 = torch.randn(B, H, 64, 64, device="cuda") * 0.1
+    y0, st0, _ = ops.forward_raw(*x, u, 64, s_in=s0, want_state=True)
+    y1, st1 = RWKVKernelOperator(64, T, segments="whole")(*x, u, return_state=True, init_state=s0)
+    assert torch.equal(y0, y1) and torch.equal(st0, st1)
