@@ -3,8 +3,9 @@ model (rwkv6_model.py): EmbeddingLayer (:219-239), RWKV_Block (:197-215: x + Tim
 TimeMix (:116-196), ChannelMix (:48-83), OutputLayer (:240-259), RWKV6 (:260-276).
 
 Hand-written kernels: the WKV recurrence (``ops.wkv6``), the token-shift interpolations in front of the projections
-(``time_mix_inputs``), the per-head GroupNorm + gate behind it (``group_norm``) and the layer norms with the residual
-additions in front of them (``layer_norm``).  The dense projections and the embedding are library calls (cuBLAS / ATen).  Used by ``bench.py --workload train_step`` and
+(``time_mix_inputs``), the per-head GroupNorm + gate behind it (``group_norm``) and, in prompt passes and token steps, the layer
+norms with the residual additions in front of them (``layer_norm``).  The dense projections and the embedding are library calls
+(cuBLAS / ATen).  Used by ``bench.py --workload train_step`` and
 ``tests/test_gpu_model.py``; weights are random (no checkpoint can be loaded here).
 """
 from __future__ import annotations
@@ -213,9 +214,10 @@ class Block(nn.Module):
         self.channel_mix = ChannelMix(hidden_size, expand_size)
 
     def forward(self, x):
-        x, h = residual_layer_norm(x, None, self.layer_norm_att)
-        x, h = residual_layer_norm(x, self.time_mix(h), self.layer_norm_ffn)
-        return x + self.channel_mix(h)
+        # norms as the framework's operations: the gradients of a step follow single rounding steps of bf16 (see TimeMix.forward), and
+        # the kernel of ``layer_norm`` rounds other elements (one in ten thousand forward, every residual gradient once instead of twice)
+        x = x + self.time_mix(self.layer_norm_att(x))
+        return x + self.channel_mix(self.layer_norm_ffn(x))
 
     @torch.no_grad()
     def prefill(self, x):
@@ -251,14 +253,14 @@ class RWKV6(nn.Module):
     def forward(self, tokens, checkpoint_blocks: bool = False):
         """``checkpoint_blocks``: keep only each block's input for the backward and recompute the block there (a
         24-layer, 2048-wide model at 32 k tokens per step would otherwise hold about 6 GB of activations per block)."""
-        x = layer_norm(self.embedding(tokens), self.embedding_ln)
+        x = self.embedding_ln(self.embedding(tokens))
         for blk in self.blocks:
             if checkpoint_blocks and torch.is_grad_enabled():
                 from torch.utils.checkpoint import checkpoint
                 x = checkpoint(blk, x, use_reentrant=False)
             else:
                 x = blk(x)
-        return self.output_layer(layer_norm(x, self.output_ln))
+        return self.output_layer(self.output_ln(x))
 
     @torch.no_grad()
     def prefill(self, tokens):

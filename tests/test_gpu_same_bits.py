@@ -106,3 +106,43 @@ def test_time_mix_walks_sequences_in_one_piece():
         model.wkv6 = wkv6
     for p, q in zip(got, want):
         assert torch.equal(p, q)
+
+
+def test_model_step():
+    """Loss and gradients of the whole model against the same modules composed of the general operations: framework norms and
+    additions, uncut recurrence, batched low-rank product, one vector mix at a time."""
+    from star_rwkv6_b200 import model, time_mix_inputs as tmi
+    from star_rwkv6_b200.loss import lm_loss
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        m = model.RWKV6(2, 512, 256, decomposer_size=32, expand_size=512, decay_rank=32).to_bf16_()
+        with torch.no_grad():
+            for blk in m.blocks:
+                blk.time_mix.mix_inputs.bias_b.normal_(0.0, 0.3)
+    tok = torch.randint(0, 512, (1, 334), device="cuda")
+    params = dict(m.named_parameters())
+
+    def step(logits):
+        loss = lm_loss(logits, tok[:, 1:])
+        return (loss, *torch.autograd.grad(loss, list(params.values())))
+
+    def general(tokens):
+        x = m.embedding_ln(m.embedding(tokens))
+        for blk in m.blocks:
+            tm, cm = blk.time_mix, blk.channel_mix
+            h = blk.layer_norm_att(x)
+            mi, (B, T, D) = tm.mix_inputs, h.shape
+            low = torch.tanh(tmi.shift_mix_vector(h, mi.time_mix_x).reshape(B * T, D) @ mi.dense_a).reshape(B * T, 5, -1).transpose(0, 1)
+            l = torch.baddbmm(mi.bias_b, low, mi.dense_b)
+            xr, xk, xv, xw, xg = tmi.shift_mix_tensors(h, l.reshape(5, B, T, D))
+            w = tm.w_b(torch.tanh(tm.w_a(xw)))
+            y, _ = torch.ops.wkv6_b200.forward(tm.dense_r(xr), tm.dense_k(xk), tm.dense_v(xv), w, tm.time_faaaa, 64, True, 0)
+            x = x + tm.dense_o(tm.group_norm(y, tm.dense_g(xg), gate_is_raw=True))
+            h = blk.layer_norm_ffn(x)
+            k = model.relu_sq(cm.dense_key(tmi.shift_mix_vector(h, cm.time_mix_k)))
+            x = x + model.sigmoid_mul(cm.dense_receptance(tmi.shift_mix_vector(h, cm.time_mix_r)), cm.dense_value(k))
+        return m.output_layer(m.output_ln(x))
+
+    got, want = step(m(tok[:, :-1])), step(general(tok[:, :-1]))
+    for name, p, q in zip(("loss", *params), got, want):
+        assert torch.equal(p, q), name
