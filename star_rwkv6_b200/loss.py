@@ -31,11 +31,13 @@ class _LMLoss(torch.autograd.Function):
         return loss_rows.mean()
 
     @staticmethod
+    @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
         (g,) = ctx.saved_tensors
         scale = grad_out.to(torch.float32)
         with torch.cuda.device(g.device):      # in place: the buffer is this function's own; nothing moves for a factor of 1
             check(lib.wkv6_scale_bf16(g.numel(), _ptr(g), _ptr(scale), _stream(g.device)))
+        torch.autograd.graph.increment_version(g)      # a second backward would scale it again: autograd refuses that
         return g.view(ctx.shape), None
 
 

@@ -60,3 +60,25 @@ def test_lm_loss_falls_back_for_other_shapes():
     rows = torch.nn.functional.cross_entropy(logits.float(), masked.clamp(0, 12), reduction="none")
     want = (rows[0] + rows[2]) / 4
     assert abs(lm_loss(logits, masked).item() - want.item()) <= 1e-6
+
+
+@pytest.mark.parametrize("factor", [0.5, 1.0])
+def test_second_backward_is_refused(factor):
+    """The backward scales the gradient in the buffer it is saved in: a second one through a retained graph must not scale it again."""
+    from star_rwkv6_b200.loss import lm_loss
+    z = torch.randn(4, 64, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    loss = lm_loss(z * 1, torch.tensor([1, 5, 63, 0], device="cuda")) * factor
+    (first,) = torch.autograd.grad(loss, z, retain_graph=True)
+    kept = first.clone()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(loss, z)
+    assert torch.equal(first, kept)
+
+
+def test_derivative_of_the_gradient_is_refused():
+    from star_rwkv6_b200.loss import lm_loss
+    z = torch.randn(4, 64, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    s = torch.tensor(0.5, device="cuda", requires_grad=True)
+    with pytest.raises(RuntimeError):
+        (g,) = torch.autograd.grad(lm_loss(z * 1, torch.tensor([1, 5, 63, 0], device="cuda")) * s, z, create_graph=True)
+        torch.autograd.grad(g.float().sum(), s)
