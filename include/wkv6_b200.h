@@ -96,7 +96,8 @@ WKV6_API int wkv6_resolve_variant(const wkv6_problem *p);
  *   s_map  : optional int64[B] device array, row b starts from s_in[s_map[b]]; NULL = identity when
  *            s_kinds == B, all-zero when s_kinds == 1.  Values must lie in [0, s_kinds): the caller
  *            validates them (the kernel clamps instead of trapping).
- *   s_out  : optional [B, H, N, N] final states
+ *   s_out  : optional [B, H, N, N] final states (may be s_in where row b starts from state b)
+ *   r, k, v, w and y lie at 16-byte boundaries; u, s_in and s_out anywhere that suits their type.
  *   ckpt   : optional checkpoint buffer of wkv6_ckpt_bytes(p) bytes.  When given, the forward stores what
  *            the backward of the same variant needs so that it does not recompute it.
  */

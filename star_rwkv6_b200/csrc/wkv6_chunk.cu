@@ -381,12 +381,12 @@ int chunk_backward_split(const wkv6_problem *p, const Dims &d, const void *r, co
 //   forward : S_in[g] = state entering segment g      = 2^{dec[g-1]} S_in[g-1] + b[g-1],  S_in[0] = s0 (or 0)
 //   reverse : A_in[g] = reverse state entering at the end of segment g = 2^{dec[g+1]} A_in[g+1] + b[g+1],  A_in[G-1] = 0
 // Segment g of sequence (b, h) sits at batch index b*G + g of the [B*G, H, ...] summary arrays.
-// A thread carries four neighbouring elements of one state row.
+// A thread carries four neighbouring elements of one state row (vec: the summaries and results lie at a 16-byte boundary).
 __global__ void __launch_bounds__(128) state_scan_kernel(int B, int H, int G, const float *__restrict__ dec,
                                                          const float *__restrict__ bsum, const void *__restrict__ s0,
                                                          const int64_t *__restrict__ s_map, int s_kinds, int s_dtype,
                                                          float *__restrict__ out, void *__restrict__ last, int last_dtype,
-                                                         bool reverse) {
+                                                         bool reverse, bool vec) {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over B*H*64*16
     if (idx >= (size_t)B * H * 1024) return;
     const int ij = (int)(idx & 1023) * 4, i = ij >> 6;
@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(128) state_scan_kernel(int B, int H, int G, co
             if (gg < G) {
                 const size_t seq = ((size_t)(b * G + (reverse ? G - 1 - gg : gg)) * H + h);
                 d8[e] = dec[seq * 64 + i];
-                b8[e] = *reinterpret_cast<const float4 *>(bsum + seq * 4096 + ij);
+                const float *p = bsum + seq * 4096 + ij;
+                b8[e] = vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
             }
         }
 #pragma unroll
@@ -417,7 +418,9 @@ __global__ void __launch_bounds__(128) state_scan_kernel(int B, int H, int G, co
             const int gg = g0 + e;
             if (gg < G) {
                 const size_t seq = ((size_t)(b * G + (reverse ? G - 1 - gg : gg)) * H + h);
-                *reinterpret_cast<float4 *>(out + seq * 4096 + ij) = make_float4(s[0], s[1], s[2], s[3]);
+                float *p = out + seq * 4096 + ij;
+                if (vec) *reinterpret_cast<float4 *>(p) = make_float4(s[0], s[1], s[2], s[3]);
+                else { p[0] = s[0]; p[1] = s[1]; p[2] = s[2]; p[3] = s[3]; }
                 const float d = exp2f(d8[e]);
                 s[0] = fmaf(d, s[0], b8[e].x); s[1] = fmaf(d, s[1], b8[e].y);
                 s[2] = fmaf(d, s[2], b8[e].z); s[3] = fmaf(d, s[3], b8[e].w);
@@ -435,7 +438,7 @@ int state_scan(int B, int H, int G, const float *dec, const float *bsum, const v
     const size_t n = (size_t)B * H * 1024;
     if (n == 0 || G <= 0) return WKV6_OK;
     state_scan_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(B, H, G, dec, bsum, s0, s_map, s_kinds, s_dtype, out, last,
-                                                                   last_dtype, reverse);
+                                                                   last_dtype, reverse, aligned16(bsum) && aligned16(out));
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? WKV6_OK : cuda_fail(e, "state_scan_kernel launch");
 }

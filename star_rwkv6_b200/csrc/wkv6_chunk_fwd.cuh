@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
     // u of this thread's channel pair (requested before the state so that the two reads overlap)
     float2 u2 = make_float2(0.f, 0.f);
     if (a.u != nullptr) {
-        if (a.u_dtype == WKV6_F32) u2 = *reinterpret_cast<const float2 *>(static_cast<const float *>(a.u) + (size_t)h * 64 + 2 * lane);
+        if (a.u_dtype == WKV6_F32 && (reinterpret_cast<uintptr_t>(a.u) & 7) == 0) u2 = *reinterpret_cast<const float2 *>(static_cast<const float *>(a.u) + (size_t)h * 64 + 2 * lane);
         else u2 = make_float2(load_any(a.u, a.u_dtype, (size_t)h * 64 + 2 * lane), load_any(a.u, a.u_dtype, (size_t)h * 64 + 2 * lane + 1));
     }
     // state in accumulator-fragment layout: rows i = ta (+8), columns j = 8(n0+nn) + 2q (+1)
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256, 2) chunk_fwd_kernel(const __grid_constant
             kind = kind < 0 ? 0 : (kind >= a.s_kinds ? a.s_kinds - 1 : kind);
             so = ((size_t)kind * a.H + h) * 4096;
         }
-        if (has && a.s_dtype == WKV6_F32) {
+        if (has && a.s_dtype == WKV6_F32 && (reinterpret_cast<uintptr_t>(a.s_in) & 7) == 0) {   // callers' states may lie anywhere
             // eight independent 8-byte loads per thread (the generic reader below switches on the dtype per element,
             // which serialises its sixteen loads: 5 us of a launch over short sequences)
             const float *sp = static_cast<const float *>(a.s_in) + so;

@@ -17,6 +17,7 @@ struct Dims {
 };
 
 int sm_count();   // of the current device
+inline bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t e, const char *what);
 size_t dtype_size(int dt);

@@ -211,6 +211,8 @@ int seq_forward(const wkv6_problem *p, const Dims &d, const void *r, const void 
         StepFwdArgs a = step_fwd_args(p, step_geom(p, d, 1, p->T));
         a.P = r; a.Q = k; a.W = w; a.X = v; a.u = u; a.out = y;
         a.s_in = s_in; a.s_map = s_map; a.s_kinds = s_kinds; a.s_out = s_out;
+        a.vec_in = p->s_dtype == WKV6_F32 && aligned16(s_in);
+        a.vec_out = p->s_dtype == WKV6_F32 && aligned16(s_out);
         return step_forward(p, a, st);
     }
     SeqColArgs a{};

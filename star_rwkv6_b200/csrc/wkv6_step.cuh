@@ -158,6 +158,7 @@ struct StepFwdArgs {
     void *s_out;                 // G == 1: optional final state
     float *b_out, *dec_out;      // summary: state built from zero [B*G,H,64,64], log2 of the total decay [B*G,H,64]
     int skip_g;                  // summary: the segment no scan reads (-1: none)
+    bool vec_in, vec_out;        // s_in / s_out are fp32 at a 16-byte boundary: 128-bit accesses (callers' states may lie anywhere)
     StepGeom q;
 };
 
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_kernel(const StepFwdArg
         int64_t kind = a.s_map ? a.s_map[s.b] : (a.s_kinds == 1 ? 0 : s.b);
         kind = kind < 0 ? 0 : (kind >= a.s_kinds ? a.s_kinds - 1 : kind);
         const size_t so = ((size_t)kind * a.q.H + s.h) * 4096;
-        if (a.s_dtype == WKV6_F32) {
+        if (a.vec_in) {
             load_tile(static_cast<const float *>(a.s_in) + so, ti, tj, S);
         } else {
 #pragma unroll
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_kernel(const StepFwdArg
     void *so = SUMMARY ? (void *)a.b_out : a.s_out;
     if (so != nullptr) {
         const int dt = SUMMARY ? (int)WKV6_F32 : a.s_dtype;
+        const bool vec = SUMMARY || a.vec_out;
 #pragma unroll
         for (int p = 0; p < 4; ++p)
 #pragma unroll
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_kernel(const StepFwdArg
                 const float2 v0 = f2_unpack(S[p][4 * half]), v1 = f2_unpack(S[p][4 * half + 1]);
                 const float2 v2 = f2_unpack(S[p][4 * half + 2]), v3 = f2_unpack(S[p][4 * half + 3]);
                 const size_t o = s.seq * 4096 + (size_t)tile_index(ti, 2 * p) * 64 + 32 * half + 4 * tj;
-                if (dt == WKV6_F32) {
+                if (vec) {
                     float *f = static_cast<float *>(so) + o;
                     *reinterpret_cast<float4 *>(f) = make_float4(v0.x, v1.x, v2.x, v3.x);
                     *reinterpret_cast<float4 *>(f + 64) = make_float4(v0.y, v1.y, v2.y, v3.y);
