@@ -136,6 +136,7 @@ WKV6_API size_t wkv6_backward_workspace_bytes(const wkv6_problem *p, int have_ck
  *   workspace : wkv6_split_workspace_bytes(p, 0 forward / 1 backward) bytes of device scratch
  *   gu_rows   : fp32 [B*G, H, N]; gu is their sum over the first axis (wkv6_sum_rows).  Order: [B][G] (sequential variant) or
  *               [G][B] (chunked variant)
+ * s_in and s_out must not overlap in the chunked variant (WKV6_ERR_INVALID).
  * The backward of fp16 inputs is not split (WKV6_ERR_UNSUPPORTED): use wkv6_backward for it.
  * No counterpart in the reference (its kernels walk each sequence with one block).
  */

@@ -215,9 +215,15 @@ int wkv6_forward_split(const wkv6_problem *p, const void *r, const void *k, cons
     if (s_in == nullptr && s_map != nullptr) return fail(WKV6_ERR_INVALID, "s_map given without s_in");
     if (s_in != nullptr && (s_kinds < 1 || s_kinds > p->B || (s_map == nullptr && s_kinds != 1 && s_kinds != p->B)))
         return fail(WKV6_ERR_INVALID, "s_kinds=%d does not fit B=%d", s_kinds, p->B);
-    if (resolve_variant(p) == WKV6_VARIANT_CHUNK)
+    if (resolve_variant(p) == WKV6_VARIANT_CHUNK) {
+        // the segments of a sequence read s_in on their own while its last one writes s_out
+        const uintptr_t in = reinterpret_cast<uintptr_t>(s_in), out = reinterpret_cast<uintptr_t>(s_out);
+        const size_t each = (size_t)p->H * p->N * p->N * dtype_size(p->s_dtype);
+        if (s_in != nullptr && s_out != nullptr && in < out + p->B * each && out < in + s_kinds * each)
+            return fail(WKV6_ERR_INVALID, "s_in and s_out overlap: not possible with cut sequences of the chunked variant");
         return chunk_forward_split(p, d, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, states, static_cast<float *>(workspace),
                                    static_cast<cudaStream_t>(stream));
+    }
     return seq_forward_split(p, d, G, r, k, v, w, u, y, s_in, s_map, s_kinds, s_out, states, static_cast<float *>(workspace),
                              static_cast<cudaStream_t>(stream));
 }

@@ -125,3 +125,15 @@ def test_product_never_touches_the_oracle():
                 text = open(os.path.join(dirpath, f), errors="ignore").read()
                 assert not re.search(r"^\s*(from|import)\s+oracle\b", text, re.M), f
                 assert "libwkv6_oracle" not in text and "oracle/" not in text, f
+
+
+def test_cut_forward_refuses_states_in_place(L):
+    """Segments of a cut sequence read the initial state on their own while the last one writes the final state."""
+    lib = L.lib
+    p = _problem(L, B=2, T=1024, H=2, x_dtype=L.BF16, y_dtype=L.BF16)
+    assert lib.wkv6_split_segments(ctypes.byref(p)) > 1
+    ws = lib.wkv6_split_workspace_bytes(ctypes.byref(p), 0)
+    a, each = 0x100000, 2 * 64 * 64 * 4
+    for s_out in (a, a + each, a - each):
+        assert lib.wkv6_forward_split(ctypes.byref(p), a, a, a, a, a, a, a, None, 2, s_out, None, a, ws, None) == -1
+        assert b"overlap" in lib.wkv6_last_error()
