@@ -13,6 +13,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/Exceptions.h>
 #include <ATen/ATen.h>
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -63,15 +64,16 @@ bool plain_mode() {
            !torch::jit::tracer::isTracing();
 }
 
-// A strided CUDA tensor of the exact class Tensor (or Parameter), not wrapped by a functorch transform.
-bool plain_tensor(PyObject *o) {
-    if (!THPVariable_CheckExact(o)) return false;
-    const Tensor &t = THPVariable_Unpack(o);
-    constexpr c10::DispatchKeySet odd({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+// A strided CUDA tensor that is what its memory holds: not wrapped by a transform, no lazy negation.
+bool plain_storage(const Tensor &t) {
+    constexpr c10::DispatchKeySet odd({c10::DispatchKey::Python, c10::DispatchKey::Batched, c10::DispatchKey::FuncTorchBatched,
                                        c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
                                        c10::DispatchKey::Conjugate, c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
-    return t.defined() && t.is_cuda() && t.layout() == at::kStrided && (t.key_set() & odd).empty();
+    return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.has_storage() && (t.key_set() & odd).empty();
 }
+
+// ... and of the exact class Tensor (or Parameter).
+bool plain_tensor(PyObject *o) { return THPVariable_CheckExact(o) && plain_storage(THPVariable_Unpack(o)); }
 
 struct Call {
     wkv6_problem p{};
@@ -164,6 +166,20 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
         return y;
     }
 
+    // Gradients that are batched (is_grads_batched, vectorised Jacobians), lazily negated or of another class: the registered
+    // operator, whose dispatch takes them apart.  The chunked variant's kept states are the checkpoints it expects; its sequential
+    // variant expects none.
+    static variable_list through_dispatcher(const Call &c, const variable_list &s, const Tensor &gy) {
+        static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("wkv6_b200::backward", "").typed<std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>(
+            const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, int64_t, int64_t)>();
+        const Tensor &r = s[0], &u = s[4];
+        auto [gr, gk, gv, gw, rows] = op.call(r, s[1], s[2], s[3], u, gy, c.chunked ? s[5] : bytes(0, r), c.p.N, c.p.variant);
+        const auto xt = r.scalar_type();
+        variable_list out{gr.to(xt), gk.to(xt), gv.to(xt), gw.to(xt), rows.sum(0).to(u.scalar_type()).reshape(u.sizes())};
+        out.resize(8);
+        return out;
+    }
+
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         variable_list s = ctx->get_saved_variables();
         const Tensor &r = s[0], &k = s[1], &v = s[2], &w = s[3], &u = s[4], &kept = s[5];
@@ -177,6 +193,7 @@ struct WKV6Function : public torch::autograd::Function<WKV6Function> {
                                   ctx->saved_data["cut"].toBool(), c),
                         "wkv6: unsupported call");
             Tensor gy = grads[0];
+            if (!plain_storage(gy)) return through_dispatcher(c, s, gy);
             if (gy.strides() != r.strides() || reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 != 0)
                 gy = like(r, c.yt, c.dense).copy_(gy);
             gr = like(r, c.yt, c.dense); gk = like(r, c.yt, c.dense);

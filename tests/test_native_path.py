@@ -81,3 +81,22 @@ def test_cut_and_whole_sequences(B, T, H, dtype, tol):
     y0, st0, _ = ops.forward_raw(*x, u, 64, s_in=s0, want_state=True)
     y1, st1 = RWKVKernelOperator(64, T, segments="whole")(*x, u, return_state=True, init_state=s0)
     assert torch.equal(y0, y1) and torch.equal(st0, st1)
+
+
+@pytest.mark.parametrize("B,T,H,dtype", [(2, 70, 2, torch.bfloat16), (1, 300, 2, torch.bfloat16), (2, 33, 2, torch.float32), (1, 130, 2, torch.float32),
+                                         (1, 40, 1, torch.float16)])
+def test_incoming_gradients_that_are_not_plain(B, T, H, dtype):
+    """Batched gradients and a lazily negated one give what plain ones give (to rounding: the custom op is never cut)."""
+    from star_rwkv6_b200 import ops
+    x, u, _ = _inputs(B, T, H, 64, dtype, 9)
+    leaves = [t.requires_grad_(True) for t in (*x, u)]
+    gys = torch.randn(3, B, T, H * 64, device="cuda").to(ops.out_dtype(dtype))
+    y = ops.wkv6(*leaves, 64)
+    want = [torch.autograd.grad(y, leaves, g, retain_graph=True) for g in gys]
+    got = torch.autograd.grad(y, leaves, gys, is_grads_batched=True, retain_graph=True)
+    neg = torch.autograd.grad(y, leaves, torch._neg_view(-gys[0]), retain_graph=True)
+    tol = 2e-2 if dtype == torch.bfloat16 else 2e-3 if dtype == torch.float16 else 2e-5
+    for i, name in enumerate(("gr", "gk", "gv", "gw", "gu")):
+        for a, b in [(got[i][j], want[j][i]) for j in range(3)] + [(neg[i], want[0][i])]:
+            assert a.shape == b.shape and a.dtype == b.dtype
+            assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm()), name
