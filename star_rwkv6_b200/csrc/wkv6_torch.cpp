@@ -102,13 +102,17 @@ bool make_call(const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &
     if (u.device() != dev || (u.scalar_type() != c.xt && u.scalar_type() != at::kFloat) || u.numel() != c.C || !u.is_contiguous())
         return false;
     if (dtype_code(c.xt) < 0 || r.stride(2) != 1) return false;
+    // rows that overlap (broadcast inputs, windows): outputs have the inputs' strides, and the C ABI takes a stride of 0 for "dense"
+    const int64_t ld = c.T > 1 ? r.stride(1) : c.C, bs = c.B > 1 ? r.stride(0) : c.T * ld;
+    if (c.T > 1 && ld < c.C) return false;
+    if (c.B > 1 && bs < (c.T - 1) * ld + c.C && (bs < c.C || (c.T > 1 && ld < (c.B - 1) * bs + c.C))) return false;
     c.dense = r.is_contiguous();
     wkv6_problem &p = c.p;
     p.B = (int32_t)c.B; p.T = (int32_t)c.T; p.H = (int32_t)c.H; p.N = (int32_t)N;
     p.x_dtype = dtype_code(c.xt); p.y_dtype = dtype_code(c.yt); p.u_dtype = dtype_code(u.scalar_type());
     p.gu_dtype = WKV6_F32; p.s_dtype = WKV6_F32; p.variant = (int32_t)variant;
-    p.row_stride = c.T > 1 ? r.stride(1) : c.C;
-    p.batch_stride = c.B > 1 ? r.stride(0) : c.T * p.row_stride;
+    p.row_stride = ld;
+    p.batch_stride = bs;
     const int variant_of = api.resolve_variant(&p);
     if (variant_of < 0) return false;
     c.chunked = variant_of == WKV6_VARIANT_CHUNK;

@@ -65,6 +65,22 @@ def _out_like(ref: torch.Tensor, dtype) -> torch.Tensor:
     return torch.empty_strided(ref.shape, ref.stride(), dtype=dtype, device=ref.device)
 
 
+def _rows_apart(t: torch.Tensor) -> bool:
+    """Whether no two rows of a [B,T,C] tensor share memory (broadcast and windowed views do: outputs could not have their strides)."""
+    B, T, C = t.shape
+    ld, bs = _strides(t)
+    if B == 0 or T == 0 or C == 0:
+        return True
+    if T > 1 and ld < C:
+        return False
+    return B == 1 or bs >= (T - 1) * ld + C or (bs >= C and (T == 1 or ld >= (B - 1) * bs + C))
+
+
+def _apart(*ts: torch.Tensor):
+    """Inputs as they are, or dense copies where rows overlap."""
+    return ts if all(_rows_apart(t) for t in ts) else tuple(t.contiguous() for t in ts)
+
+
 def _same_layout(ref: torch.Tensor, *others: torch.Tensor) -> None:
     for o in others:
         assert o.shape == ref.shape and o.stride() == ref.stride(), "r, k, v, w (and gy) must share one layout"
@@ -96,6 +112,7 @@ def forward_raw(r, k, v, w, u, head_size: int, *, s_in=None, s_map=None, want_st
                 variant: int = _lib.VARIANT_AUTO):
     """Launch the forward.  Returns (y, s_out or None, ckpt or None)."""
     _check_cuda(r, k, v, w, u, s_in, s_map)
+    r, k, v, w = _apart(r, k, v, w)
     _same_layout(r, k, v, w)
     B, T, C = r.shape
     H, N = C // head_size, head_size
@@ -133,6 +150,7 @@ def forward_raw(r, k, v, w, u, head_size: int, *, s_in=None, s_map=None, want_st
 def backward_raw(r, k, v, w, u, gy, head_size: int, *, ckpt=None, variant: int = _lib.VARIANT_AUTO):
     """Launch the backward.  Returns (gr, gk, gv, gw, gu[B,H,N] fp32)."""
     _check_cuda(r, k, v, w, u, gy, ckpt)
+    r, k, v, w = _apart(r, k, v, w)
     _same_layout(r, k, v, w)
     B, T, C = r.shape
     H, N = C // head_size, head_size
@@ -160,6 +178,7 @@ def wkv6_decode(r, k, v, w, u, head_size: int, state=None, state_map=None, out_s
     _check_cuda(r, k, v, w, u, state, state_map, out_state)
     B, T, C = r.shape
     assert T == 1 and head_size == 64 and r.is_contiguous()
+    k, v, w = (t.contiguous() for t in (k, v, w))      # the kernel reads all four densely
     H = C // head_size
     ydt = out_dtype(r.dtype)
     p = make_problem(r, u, head_size, ydt, _lib.VARIANT_AUTO)
