@@ -46,8 +46,8 @@ class _ResidualLayerNorm(torch.autograd.Function):
             return gs, (gs if ctx.has_o else None), None, None, None
         D = s.shape[-1]
         rows = s.numel() // D
-        gy = gy.contiguous()
-        gs = None if gs is None else gs.contiguous()
+        gy = _dense16(gy)
+        gs = None if gs is None else _dense16(gs)
         gx, gg, gb = torch.empty_like(s), torch.empty_like(gamma), torch.empty_like(gamma)
         nbytes = lib.wkv6_layer_norm_workspace_bytes(rows, D)
         ws = torch.empty((max(nbytes, 16),), dtype=torch.uint8, device=s.device)
@@ -57,20 +57,36 @@ class _ResidualLayerNorm(torch.autograd.Function):
         return gx, (gx if ctx.has_o else None), gg, gb, None
 
 
+def _own_forward(module, cls) -> bool:
+    """Whether calling ``module`` does what ``cls`` does and nothing else: no subclass, no hooks on it or on all modules."""
+    m = torch.nn.modules.module
+    return (type(module) is cls
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+            and not (m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks))
+
+
 def _fits(x, ln):
+    """Whether the kernel covers ln(x): otherwise the framework's operations run (and raise, where they do)."""
+    if not _own_forward(ln, nn.LayerNorm) or not x.is_cuda or x.dtype != torch.bfloat16 or x.numel() == 0:
+        return False
     D = x.shape[-1]
-    return (x.is_cuda and x.dtype == torch.bfloat16 and D % 8 == 0 and D <= MAX_CHANNELS and x.numel() > 0
-            and ln.weight is not None and ln.bias is not None and ln.weight.dtype == ln.bias.dtype == torch.bfloat16
-            and ln.weight.is_contiguous() and ln.bias.is_contiguous() and tuple(ln.normalized_shape) == (D,)
-            and not (ln._forward_hooks or ln._forward_pre_hooks or ln._backward_hooks or ln._backward_pre_hooks)
+    return (D % 8 == 0 and D <= MAX_CHANNELS and tuple(ln.normalized_shape) == (D,)
+            and all(p is not None and p.dtype == torch.bfloat16 and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0
+                    for p in (ln.weight, ln.bias))
             and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda"))
+
+
+def _dense16(t):
+    """t dense and at a 16-byte boundary (a copy where it is not)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def residual_layer_norm(x, o, ln: nn.LayerNorm):
     """(s, ln(s)) with s = x + o (o None: s = x), differentiable.  bf16 tensors and parameters go through the kernel above,
     everything else through the framework's operations."""
     ts = (x,) if o is None else (x, o)
-    if not all(_fits(t, ln) and t.data_ptr() % 16 == 0 for t in ts) or (o is not None and o.shape != x.shape):
+    if not all(_fits(t, ln) and t.data_ptr() % 16 == 0 for t in ts) or (o is not None and (o.shape != x.shape or o.device != x.device)):
         s = x if o is None else x + o
         return s, ln(s)
     if torch.is_grad_enabled() and any(t.requires_grad for t in (*ts, ln.weight, ln.bias)):

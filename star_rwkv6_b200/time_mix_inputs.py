@@ -17,6 +17,7 @@ import ctypes
 import torch
 
 from ._lib import check, lib
+from .layer_norm import _dense16
 from .ops import _DT, _check_cuda, _ptr, _stream
 
 
@@ -136,7 +137,7 @@ class _LoraMix(torch.autograd.Function):
     def backward(ctx, *gout):
         x, h, wb, bias = ctx.saved_tensors
         B, T, C = x.shape
-        gout = [g.contiguous() for g in (gout[0] if ctx.stacked else gout)]
+        gout = [_dense16(g) for g in (gout[0] if ctx.stacked else gout)]
         gx = torch.empty_like(x)
         gl = torch.empty((5, B * T, C), dtype=x.dtype, device=x.device)
         with torch.cuda.device(x.device):
@@ -149,7 +150,7 @@ class _LoraMix(torch.autograd.Function):
 
 def _lora_fits(x, h, wb, bias):
     return (x.is_cuda and x.dim() == 3 and x.numel() > 0 and x.shape[-1] % 8 == 0 and wb.shape == (5, 32, x.shape[-1])
-            and all(t.dtype == torch.bfloat16 for t in (x, h, wb, bias))
+            and all(t.dtype == torch.bfloat16 and t.device == x.device for t in (x, h, wb, bias))
             and all(t.data_ptr() % 16 == 0 for t in (x, h, wb, bias)))
 
 
