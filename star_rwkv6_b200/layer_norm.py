@@ -60,7 +60,7 @@ class _ResidualLayerNorm(torch.autograd.Function):
 def _own_forward(module, cls) -> bool:
     """Whether calling ``module`` does what ``cls`` does and nothing else: no subclass, no hooks on it or on all modules."""
     m = torch.nn.modules.module
-    return (type(module) is cls
+    return (type(module) is cls and "forward" not in module.__dict__
             and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
             and not (m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks))
 

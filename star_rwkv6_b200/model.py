@@ -17,7 +17,7 @@ from . import decode_stages as ds
 from .channel_mix_ops import relu_sq, sigmoid_mul
 from .group_norm import GroupNormGate
 from .group_norm import groupnorm_gate_forward_raw
-from .layer_norm import layer_norm, residual_layer_norm
+from .layer_norm import _own_forward, layer_norm, residual_layer_norm
 from .ops import wkv6, wkv6_decode, wkv6_with_state
 from .time_mix_inputs import TimeMixInputs, shift_mix_pair
 
@@ -80,8 +80,13 @@ class TimeMix(nn.Module):
         with torch.no_grad():
             self.w_b.bias.uniform_(-6.0, -1.0)  # decays exp(-exp(w)) spread between slow and fast channels
 
+    def _mixed(self, x):
+        """The five mixed inputs.  Five tensors without the stack in between, where nothing listens to the module's call."""
+        mi = self.mix_inputs
+        return mi.split(x) if _own_forward(mi, TimeMixInputs) else mi(x)
+
     def forward(self, x):
-        xr, xk, xv, xw, xg = self.mix_inputs.split(x)
+        xr, xk, xv, xw, xg = self._mixed(x)
         r, k, v = self.dense_r(xr), self.dense_k(xk), self.dense_v(xv)
         w = self.w_b(torch.tanh(self.w_a(xw)))
         # in one piece: the per-head norm behind it magnifies single rounding steps of y into percents of the gradients, so a row's
@@ -97,7 +102,7 @@ class TimeMix(nn.Module):
     @torch.no_grad()
     def prefill(self, x):
         """Forward over a whole prompt; returns the output and the layer state (last input token, WKV state)."""
-        xr, xk, xv, xw, xg = self.mix_inputs.split(x)
+        xr, xk, xv, xw, xg = self._mixed(x)
         r, k, v = self.dense_r(xr), self.dense_k(xk), self.dense_v(xv)
         w = self.w_b(torch.tanh(self.w_a(xw)))
         y, S = wkv6_with_state(r, k, v, w, self.time_faaaa, self.head_size)

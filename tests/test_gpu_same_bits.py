@@ -146,3 +146,24 @@ def test_model_step():
     got, want = step(m(tok[:, :-1])), step(general(tok[:, :-1]))
     for name, p, q in zip(("loss", *params), got, want):
         assert torch.equal(p, q), name
+
+
+@pytest.mark.parametrize("how", ["hook", "subclass", "replaced"])
+def test_module_of_the_mixed_inputs_is_called(how):
+    """Hooks on the module, a forward of a subclass and a module in its place take part in the block's passes."""
+    from star_rwkv6_b200 import model
+    torch.manual_seed(0)
+    tm, seen = model.TimeMix(128).cuda(), []
+    x = torch.randn(2, 9, 128, device="cuda")
+    with torch.no_grad():
+        want, (want_prefill, _) = tm(x), tm.prefill(x)
+        mi = tm.mix_inputs
+        if how == "hook":
+            mi.register_forward_hook(lambda m, args, out: seen.append(out.shape))
+        elif how == "subclass":
+            mi.__class__ = type("Logged", (type(mi),), {"forward": lambda self, x: (seen.append(x.shape), type(self).__mro__[1].forward(self, x))[1]})
+        else:
+            tm.mix_inputs = torch.nn.Identity()
+            tm.mix_inputs.forward = lambda x: (seen.append(x.shape), mi(x))[1]
+        assert torch.equal(tm(x), want) and torch.equal(tm.prefill(x)[0], want_prefill)
+    assert len(seen) == 2
