@@ -39,11 +39,15 @@ def xla_ffi_include_dir():
 
 
 def native_command():
-    """g++ line for _native.so.  torch is located without importing it; its libraries are in the process before the
-    module is (the package imports torch first), so no run path is recorded."""
+    """g++ line for _native.so, or None where torch is not installed (a host that uses the C ABI or the JAX targets only).  torch is
+    located without importing it; its libraries are in the process before the module is (the package imports torch first), so
+    no run path is recorded."""
     import importlib.util
     import sysconfig
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    spec = importlib.util.find_spec("torch")
+    if spec is None:
+        return None
+    torch_dir = os.path.dirname(spec.origin)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
@@ -53,9 +57,10 @@ def native_command():
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(NATIVE):
+    built = [LIB] + ([NATIVE] if native_command() else [])
+    if not all(os.path.exists(f) for f in built):
         return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(NATIVE))
+    t = min(os.path.getmtime(f) for f in built)
     deps = glob.glob(os.path.join(CSRC, "*")) + glob.glob(os.path.join(PKG, "..", "include", "*.h"))
     return any(os.path.getmtime(f) > t for f in deps)
 
@@ -78,7 +83,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc, "-x", "cu"] + flags + ["-I", inc, "-c", src, "-o", obj]
         procs.append((cmd, subprocess.Popen(cmd)))
         objs.append(obj)
-    procs.append((native_command(), subprocess.Popen(native_command())))
+    if native_command():
+        procs.append((native_command(), subprocess.Popen(native_command())))
     for cmd, pr in procs:
         if pr.wait() != 0:
             raise RuntimeError("compilation failed: " + " ".join(cmd))

@@ -12,6 +12,7 @@ There is no CPU implementation: tensors that are not on a CUDA device are reject
 from __future__ import annotations
 
 import ctypes
+import warnings
 from typing import Optional, Tuple
 
 import torch
@@ -21,10 +22,15 @@ from ._lib import BF16, F16, F32, Problem, check, lib
 
 try:
     from . import _native  # csrc/wkv6_torch.cpp: the same calls without Python between the caller and the C ABI
+    _native.bind(_lib.LIB_PATH)
 except ImportError as e:
-    raise ImportError("star_rwkv6_b200/_native.so is missing or was built against another torch: build it with "
-                      "`python star_rwkv6_b200/build.py`") from e
-_native.bind(_lib.LIB_PATH)
+    # the same kernels through ctypes and the registered operators, 20 us or more slower per call, and never cut along T
+    warnings.warn(f"star_rwkv6_b200/_native.so does not load ({e}): calls take the slower Python path.  It belongs to the torch it was "
+                  "built against: `python star_rwkv6_b200/build.py` builds it for this one.", RuntimeWarning, stacklevel=2)
+
+    class _native:
+        """Leaves every call to the Python path, as the module does with calls that it does not handle."""
+        wkv6 = with_state = staticmethod(lambda *args: None)
 
 _DT = {torch.bfloat16: BF16, torch.float16: F16, torch.float32: F32}
 
