@@ -396,7 +396,8 @@ int wkv6_shift_mix_forward(int32_t B, int32_t T, int32_t C, int32_t dtype, int32
 __attribute__((visibility("default")))
 size_t wkv6_shift_mix_workspace_bytes(int32_t B, int32_t T, int32_t C, int32_t m_is_vector) {
     if (!m_is_vector || B <= 0 || T <= 0 || C <= 0) return 0;
-    return m_is_vector > 2 ? 0 : (size_t)m_is_vector * B * vec_blocks(T, m_is_vector) * C * sizeof(float);
+    const int nv = m_is_vector == 2 ? 2 : 1;     // any other value is a truth value
+    return (size_t)nv * B * vec_blocks(T, nv) * C * sizeof(float);
 }
 
 __attribute__((visibility("default")))

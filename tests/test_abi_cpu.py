@@ -137,3 +137,11 @@ def test_cut_forward_refuses_states_in_place(L):
     for s_out in (a, a + each, a - each):
         assert lib.wkv6_forward_split(ctypes.byref(p), a, a, a, a, a, a, a, None, 2, s_out, None, a, ws, None) == -1
         assert b"overlap" in lib.wkv6_last_error()
+
+
+def test_shift_mix_workspace_takes_any_truth_value(L):
+    size = L.lib.wkv6_shift_mix_workspace_bytes
+    one = size(2, 100, 64, 1)
+    assert one > 0 and size(2, 100, 64, 0) == 0
+    assert size(2, 100, 64, 3) == size(2, 100, 64, -1) == one
+    assert size(2, 100, 64, 2) >= 2 * one          # a pair of mixes
