@@ -100,3 +100,28 @@ def test_incoming_gradients_that_are_not_plain(B, T, H, dtype):
         for a, b in [(got[i][j], want[j][i]) for j in range(3)] + [(neg[i], want[0][i])]:
             assert a.shape == b.shape and a.dtype == b.dtype
             assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm()), name
+
+
+def test_cut_call_captured_on_a_side_stream():
+    """A shape that the library cuts, forward and backward in a CUDA graph: replays on new inputs have the bits of eager calls."""
+    from star_rwkv6_b200 import ops
+    x, u, gy = _inputs(1, 1003, 2, 64, torch.bfloat16, 10)
+    gy = gy.to(torch.bfloat16)
+    leaves = [t.requires_grad_(True) for t in (*x, u)]
+    call = lambda: _gradients(lambda *a: ops.wkv6(*a, 64), leaves[:4], leaves[4], gy)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        eager = call()                  # also the call outside the capture
+    torch.cuda.current_stream().wait_stream(side)
+    assert all(torch.equal(a, b) for a, b in zip(eager, call()))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    for seed in (11, 12):
+        fresh, v, _ = _inputs(1, 1003, 2, 64, torch.bfloat16, seed)
+        with torch.no_grad():
+            for a, b in zip(leaves, (*fresh, v)):
+                a.copy_(b)
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(out, call()))
